@@ -543,32 +543,6 @@ int read_n_alive(ntlp_ctx *c, int b, int *n) {
     return NTLP_OK;
 }
 
-__global__ void k_gather_d(const double *__restrict__ src, const int *__restrict__ perm,
-                           const int *__restrict__ lid, const int *__restrict__ rank, double *__restrict__ out,
-                           int n) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    int s = perm[t];
-    out[rank[lid[s]]] = src[s];
-}
-
-__global__ void k_gather_i64(const long long *__restrict__ src, const int *__restrict__ perm,
-                             const int *__restrict__ lid, const int *__restrict__ rank, long long *__restrict__ out,
-                             int n) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    int s = perm[t];
-    out[rank[lid[s]]] = src[s];
-}
-
-__global__ void k_gather_lid(const int *__restrict__ perm, const int *__restrict__ lid,
-                             const int *__restrict__ rank, int *__restrict__ out, int n) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    int s = perm[t];
-    out[rank[lid[s]]] = lid[s];
-}
-
 // the six source array pointers of a box, by value
 struct Src6 {
     double *p[6];
@@ -621,6 +595,17 @@ void phase_end(ntlp_ctx *c, int phase, cudaEvent_t a) {
     cudaEvent_t b = ev_get(c);
     cudaEventRecord(b, c->stream);
     c->recs.push_back({phase, a, b});
+}
+
+// whether kernels of this context can write p as elements of `align` bytes:
+// memory of its own device, aligned (anything else goes through a copy)
+bool on_device(ntlp_ctx *c, const void *p, size_t align) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == c->device && (uintptr_t)p % align == 0;
 }
 
 bool box_ok(ntlp_ctx *c, int b) { return c && b >= 0 && b < c->nbox; }
@@ -1147,16 +1132,28 @@ int droplets_download(ntlp_ctx *c, int b, ntlp_droplets *d) {
     if (n == 0) return NTLP_OK;
     const DevBox &B = c->box[b];
     const DevState &S = B.st[B.cur];
-    launch_rank_alive(c->box_d, b, h.rank, h.n_uploaded, c->stream);
-    const int blocks = (n + 255) / 256;
-    auto get = [&](const double *src, double *host) -> int {
-        if (!host || !src) return NTLP_OK;
-        k_gather_d<<<blocks, 256, 0, c->stream>>>(src, B.perm, S.lid, h.rank, h.staging, n);
-        CK(cudaMemcpyAsync(host, h.staging, (size_t)n * 8, cudaMemcpyDefault, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
+    // the list position of each droplet: its lid while every uploaded droplet
+    // is alive, else its rank among the living; the slot table takes the
+    // array of the sort's result, which is dead between steps
+    int *slot = B.sorted;
+    if (n != h.n_uploaded) launch_rank_alive(c->box_d, b, h.rank, h.n_uploaded, (int *)h.staging, c->stream);
+    launch_slots(B.perm, S.lid, n != h.n_uploaded ? h.rank : nullptr, slot, n, c->stream);
+    // arrays that live on this device are gathered in place, in one launch;
+    // the others one by one through the staging buffer
+    ListGather here{};
+    int rc = 0;
+    auto get = [&](const void *src, void *dst) -> int {
+        if (!dst || !src) return NTLP_OK;
+        ListGather one{};
+        const bool direct = on_device(c, dst, 8);
+        ListGather &g = direct ? here : one;
+        g.src[g.n] = (const double *)src;
+        g.dst[g.n++] = direct ? (double *)dst : h.staging;
+        if (direct) return NTLP_OK;
+        launch_gather_list(one, slot, n, c->stream);
+        CK(cudaMemcpyAsync(dst, h.staging, (size_t)n * 8, cudaMemcpyDefault, c->stream));
         return NTLP_OK;
     };
-    int rc = 0;
     for (int a = 0; a < 3; ++a) {
         rc |= get(S.x[a], d->xp[a]);
         rc |= get(S.v[a], d->vp[a]);
@@ -1171,14 +1168,13 @@ int droplets_download(ntlp_ctx *c, int b, ntlp_droplets *d) {
     rc |= get(S.qinf, d->qinf); rc |= get(S.qstar, d->qstar); rc |= get(S.Tpold, d->Tp_old);
     rc |= get(S.rold, d->radius_old); rc |= get(S.Tprhs_s, d->Tprhs_s); rc |= get(S.Tprhs_L, d->Tprhs_L);
     rc |= get(S.radrhs, d->radrhs);
+    rc |= get(S.mult, d->mult);
     if (rc) return rc;
-    if (d->mult) {
-        k_gather_i64<<<blocks, 256, 0, c->stream>>>(S.mult, B.perm, S.lid, h.rank, (long long *)h.staging, n);
-        CK(cudaMemcpyAsync(d->mult, h.staging, (size_t)n * 8, cudaMemcpyDefault, c->stream));
-    }
+    launch_gather_list(here, slot, n, c->stream);
     if (d->lid) {
-        k_gather_lid<<<blocks, 256, 0, c->stream>>>(B.perm, S.lid, h.rank, (int *)h.staging, n);
-        CK(cudaMemcpyAsync(d->lid, h.staging, (size_t)n * 4, cudaMemcpyDefault, c->stream));
+        const bool direct = on_device(c, d->lid, 4);
+        launch_gather_list_i32(S.lid, slot, direct ? d->lid : (int *)h.staging, n, c->stream);
+        if (!direct) CK(cudaMemcpyAsync(d->lid, h.staging, (size_t)n * 4, cudaMemcpyDefault, c->stream));
     }
     CK(cudaStreamSynchronize(c->stream));
     CK(cudaGetLastError());
@@ -2008,7 +2004,7 @@ int ntlp_sub_immigrants(ntlp_ctx *c, const ntlp_droplets *d) {
     if ((int64_t)n + m > h.cap)
         return fail(c, NTLP_ERR_CAPACITY, "%d + %d droplets exceed capacity %lld", n, m, (long long)h.cap);
     // existing droplets to slots m.. in list order, then the arrivals to 0..m-1
-    launch_rank_alive(c->box_d, 0, h.rank, h.n_uploaded, c->stream);
+    launch_rank_alive(c->box_d, 0, h.rank, h.n_uploaded, (int *)h.staging, c->stream);
     launch_shift_existing(c->box_d, 0, n, m, h.rank, c->stream);
     const DevState &O = c->box[0].st[1 - c->box[0].cur];
     auto up = [&](void *dst, const void *src, size_t esz) -> int {

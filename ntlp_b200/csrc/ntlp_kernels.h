@@ -113,8 +113,19 @@ void launch_keys_initial(DevBox *boxes, const Tile *tiles, int ntiles, cudaStrea
 void launch_fill_ext(const double *flow, double *ext, const DevGrid &g, cudaStream_t st);
 void launch_pack_f32(const DevBox *host_box, float4 *f4, float *fw, cudaStream_t st);
 
-// download: position of each survivor in list order
-void launch_rank_alive(DevBox *boxes, int box, int *rank_by_lid, int nlid, cudaStream_t st);
+// download: position of each survivor in list order (scratch: (nlid + 1023) / 1024 ints)
+void launch_rank_alive(DevBox *boxes, int box, int *rank_by_lid, int nlid, int *scratch, cudaStream_t st);
+// the state's slot of each list position; rank_by_lid nullptr: lid is the position
+void launch_slots(const int *perm, const int *lid, const int *rank_by_lid, int *slot, int n, cudaStream_t st);
+// dst[k][r] = src[k][slot[r]] for 8-byte values (int64 bits pass through unchanged)
+constexpr int kListArrays = 36;   // a droplet has 35 8-byte values
+struct ListGather {
+    const double *src[kListArrays];
+    double *dst[kListArrays];
+    int n;
+};
+void launch_gather_list(const ListGather &g, const int *slot, int n, cudaStream_t st);
+void launch_gather_list_i32(const int *src, const int *slot, int *dst, int n, cudaStream_t st);
 
 // x-y column subdomains (ntlp_subdomain.cu)
 // emigrants in send order (direction, then lid) by a radix sort
