@@ -62,6 +62,7 @@ struct BoxHost {
     std::vector<double> z, zz, dzw, dzu;
     std::vector<int> lut;           // level-search bucket tables (zz, then z)
     std::vector<float> rden;        // window denominators (zz, then z)
+    std::vector<double> rdep;       // deposition reciprocals (1/dzu, then 1/(dx dy dzu))
     int64_t cap = 0;
     int n_uploaded = 0;
     bool have_fields = false, have_droplets = false;
@@ -297,13 +298,14 @@ void carve_box(Carver &cv, BoxHost &h, DevBox &B, bool mixed) {
     const size_t npad = (size_t)g.nz2 * g.ny5 * g.nx5;
     const size_t n = (size_t)h.cap;
     double *zg;
-    cv.take(&zg, 2 * (size_t)g.nz2 + 2 * ((size_t)g.nnz + 3));
+    cv.take(&zg, 2 * (size_t)g.nz2 + 4 * ((size_t)g.nnz + 3));
     int *lut;
     cv.take(&lut, 2 * (size_t)kLutPerLevel * g.nz2);
     float *rden;
     cv.take(&rden, 2 * 6 * ((size_t)g.nnz + 3));
     if (cv.base) {
         B.g.z = zg; B.g.zz = zg + g.nz2; B.g.dzw = zg + 2 * g.nz2; B.g.dzu = zg + 2 * g.nz2 + (g.nnz + 3);
+        B.g.rdzu = B.g.dzu + (g.nnz + 3); B.g.rdV = B.g.rdzu + (g.nnz + 3);
         B.g.lut_zz = lut; B.g.lut_z = lut + kLutPerLevel * g.nz2;
         B.g.rden_zz = rden; B.g.rden_z = rden + 6 * (g.nnz + 3);
     }
@@ -332,14 +334,13 @@ void carve_box(Carver &cv, BoxHost &h, DevBox &B, bool mixed) {
     }
     carve_state(cv, B.st[0], n);
     carve_state(cv, B.st[1], n);
+    B.img = nullptr;
+    if (g.periodic) cv.take(&B.img, 6 * (size_t)img_count(g));
     if (mixed) {
         for (int q = 0; q < P32_N; ++q) cv.take(&B.pay32.f[q], n);
-        B.img = nullptr;
-        if (g.periodic) cv.take(&B.img, 6 * (size_t)img_count(g));
         B.cellsum = nullptr;
         if ((long long)h.cap >= (long long)kDenseRatio * g.ncells) cv.take(&B.cellsum, (size_t)g.ncells * 48);
     } else {
-        B.img = nullptr;
         B.cellsum = nullptr;
         for (int a = 0; a < 3; ++a) { cv.take(&B.pay.D[a], n); cv.take(&B.pay.V[a], n); }
         cv.take(&B.pay.T0, n); cv.take(&B.pay.H0, n); cv.take(&B.pay.E1, n); cv.take(&B.pay.E2, n);
@@ -672,11 +673,33 @@ void box_geometry(const ntlp_grid &grid, int64_t cap, DevBox &B) {
     B.cur = 0;
 }
 
-// mixed periodic boxes deposit their periodic images (ix = nnx+1, nnx+2;
-// iy = nny+1, nny+2) as nodes of the tiles, folded in by k_fold32
-void deposit_extents(DevGrid &g, bool mixed) {
-    g.dnx = g.snx + (mixed && g.periodic ? 2 : 0);
-    g.dny = g.sny + (mixed && g.periodic ? 2 : 0);
+// periodic boxes deposit their periodic images (ix = nnx+1, nnx+2;
+// iy = nny+1, nny+2) as nodes of the tiles, folded in by k_fold
+void deposit_extents(DevGrid &g) {
+    g.dnx = g.snx + (g.periodic ? 2 : 0);
+    g.dny = g.sny + (g.periodic ? 2 : 0);
+}
+
+// The reciprocals of the FP64 deposition's denominators, dx, dy, dzu(k) and
+// dx dy dzu(k) as the device forms them: each correctly rounded.  False when
+// one of them has a significand of all ones or is outside 2^-100 .. 2^100,
+// where the division by reciprocal is not exact (div_by); the deposition
+// then divides.
+bool deposit_reciprocals(const DevGrid &g, const std::vector<double> &dzu, std::vector<double> &rec) {
+    auto ok = [](double d) {
+        const uint64_t m = ntlp_bits(d) & 0x000fffffffffffffULL;
+        return d > 0x1p-100 && d < 0x1p100 && m != 0x000fffffffffffffULL;
+    };
+    const size_t n = dzu.size();
+    rec.assign(2 * n, 1.0);
+    bool all = ok(g.dx) && ok(g.dy);
+    for (size_t k = 0; k < n; ++k) {
+        const double dV = g.dx * g.dy * dzu[k];
+        all = all && ok(dzu[k]) && ok(dV);
+        rec[k] = 1.0 / dzu[k];
+        rec[n + k] = 1.0 / dV;
+    }
+    return all;
 }
 
 // an x-y column subdomain of the periodic domain (set_bounds,
@@ -759,7 +782,7 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
         const DevGrid &g = B.g;
         box_geometry(*grid, h.cap, B);
         if (sd) subdomain_geometry(*grid, *sd, B);
-        deposit_extents(B.g, mixed);
+        deposit_extents(B.g);
         Carver cv;
         carve_box(cv, h, B, mixed);
         h.arena_bytes = cv.off;
@@ -772,6 +795,8 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
         carve_box(cv2, h, B, mixed);
         level_tables(h, grid->nnz, h.lut, B.g.lut_scale, h.rden);
         B.g.nlut = kLutPerLevel * nz2;
+        double *rdep = (double *)B.g.rdzu;
+        if (!deposit_reciprocals(B.g, h.dzu, h.rdep)) B.g.rdzu = B.g.rdV = nullptr;
         if (mixed) {
             const size_t npad = (size_t)nz2 * B.g.ny5 * B.g.nx5 + 2 * kF32Guard;
             if (cudaMemsetAsync((void *)(B.f4 - kF32Guard), 0, npad * sizeof(float4), c->stream) ||
@@ -796,6 +821,7 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
             cudaMemcpyAsync((void *)B.g.zz, h.zz.data(), nz2 * 8, cudaMemcpyHostToDevice, c->stream) ||
             cudaMemcpyAsync((void *)B.g.dzw, h.dzw.data(), nz3 * 8, cudaMemcpyHostToDevice, c->stream) ||
             cudaMemcpyAsync((void *)B.g.dzu, h.dzu.data(), nz3 * 8, cudaMemcpyHostToDevice, c->stream) ||
+            cudaMemcpyAsync(rdep, h.rdep.data(), 2 * nz3 * 8, cudaMemcpyHostToDevice, c->stream) ||
             cudaMemsetAsync(B.cell_cnt, 0, sizeof(int) * (size_t)(g.ncells + 2), c->stream) ||
             cudaMemsetAsync(B.n_alive, 0, sizeof(int), c->stream) ||
             cudaMemsetAsync(B.hist, 0, sizeof(long long) * NTLP_H_STEP_KINDS * NTLP_HIST_N, c->stream) ||
@@ -1184,7 +1210,7 @@ int droplets_download(ntlp_ctx *c, int b, ntlp_droplets *d) {
 // kernels of one deposition: the tiles, plus the two cell-sum kernels when
 // a mixed box is dense
 int deposit_launches(const ntlp_ctx *c) {
-    if (c->params.precision != NTLP_PREC_MIXED) return 1;
+    if (c->params.precision != NTLP_PREC_MIXED) return 2;   // tiles, fold
     return c->any_dense ? 5 : 3;   // tiles, overflow, fold (+ cell sums, dense nodes)
 }
 
@@ -1229,7 +1255,7 @@ int launch_step(ntlp_ctx *c, int kind, int istage, double dt, int32_t it, bool w
             launch_deposit_mixed(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
                                  c->any_dense, c->overflow_list_d);
         else
-            launch_deposit64(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream);
+            launch_deposit64(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox);
         phase_end(c, PH_DEPOSIT, e0);
         c->launches += deposit_launches(c);
     }
@@ -1407,7 +1433,7 @@ int launch_coupling(ntlp_ctx *c, double dt) {
         launch_deposit_mixed(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
                              c->any_dense, c->overflow_list_d);
     else
-        launch_deposit64(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream);
+        launch_deposit64(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox);
     phase_end(c, PH_DEPOSIT, e0);
     c->launches += deposit_launches(c);
     CK(cudaGetLastError());
@@ -1484,7 +1510,7 @@ int64_t ntlp_bytes_required(int32_t nbox, const ntlp_grid *grids, const ntlp_par
         h.cap = capacities[b];
         DevBox B{};
         box_geometry(grids[b], h.cap, B);
-        deposit_extents(B.g, mixed);
+        deposit_extents(B.g);
         Carver cv;
         carve_box(cv, h, B, mixed);
         total += cv.off;

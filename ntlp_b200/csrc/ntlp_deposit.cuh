@@ -8,16 +8,18 @@
 // also receive their periodic images (ix+nnx, iy+nny), combined in the order
 // of the fold (x first, then y).
 //
-// The main kernel stages, per tile of TX x TY x TZ nodes, the droplets of
+// The tiled kernels stage, per tile of TX x TY x TZ nodes, the droplets of
 // the tile's (TX+1)(TY+1)(TZ+1) cells in shared memory (each (x, y) column of
-// cells is one contiguous range of the sorted list) and merges from there;
-// tiles touching the periodic edges, or holding more droplets than the
-// shared buffer, merge straight from global memory.  Both paths perform the
-// same operations in the same order.
+// cells is one contiguous range of the sorted list) and merge from there;
+// the periodic images (ix > nnx or iy > nny) are nodes of their own, folded in
+// by k_fold.  Tiles holding more droplets than the shared buffer (and, for
+// boxes without an image buffer, FP64 tiles on the periodic edges) merge
+// straight from global memory.  Both paths perform the same operations in the
+// same order.
 //
-// MIXED=false: each contribution is formed as the reference writes it,
+// FP64 (k_deposit64): each contribution is formed as the reference writes it,
 // ((P*wtt)/dV)*mult with wtt = wtx*wty*wtz, subtracted term by term.
-// MIXED=true: the FP32 payload (cell-relative fractions, momentum/heat/
+// Mixed (k_deposit_tiled): the FP32 payload (cell-relative fractions, momentum/heat/
 // vapour factors, mult/dV), FP32 weights, FP64 sums, grouped by cell: each
 // of the node's 8 cells sums its droplets in list order from zero (S_o),
 // and the node adds S_0 .. S_7 in order.  Deterministic, not list order;
@@ -96,20 +98,17 @@ __device__ __forceinline__ void cell_sum32(const DevBox &B, const DevParams &p, 
     }
 }
 
-// FP64: merge of up to 8 lid-sorted ranges.  Source: global memory through
-// the sorted list (STAGED false; positions index B.perm) or the
-// shared-memory stage (STAGED true; positions index the stage).
-template <bool STAGED>
-__device__ __forceinline__ void merge_ranges(const DevBox &B, const DevParams &p, const int *s_lid,
-                                             const double *s_v, int n, int pos[8], const int end[8],
-                                             const int ck[8], const int off[8], int px, int py, int pz,
+// FP64: merge of up to 8 lid-sorted ranges from global memory through the
+// sorted list (positions index B.perm)
+__device__ __forceinline__ void merge_ranges(const DevBox &B, const DevParams &p, int n, int pos[8],
+                                             const int end[8], const int ck[8], int px, int py, int pz,
                                              double acc[6]) {
     const DevGrid &g = B.g;
     for (int q = 0; q < 6; ++q) acc[q] = 0.0;
     if (n == 0) return;
     const DevState &O = B.st[B.cur];
     int head[8];
-    for (int c = 0; c < n; ++c) head[c] = STAGED ? s_lid[pos[c]] : O.lid[B.perm[pos[c]]];
+    for (int c = 0; c < n; ++c) head[c] = O.lid[B.perm[pos[c]]];
     const double xv = g.dx * (double)(px + g.ioff - 1);
     const double yv = g.dy * (double)(py + g.joff - 1);
     const double zv = g.zz[pz];
@@ -121,26 +120,91 @@ __device__ __forceinline__ void merge_ranges(const DevBox &B, const DevParams &p
         const int at = pos[best];
         const int kpt = ck[best];
         pos[best]++;
-        if (pos[best] < end[best]) head[best] = STAGED ? s_lid[pos[best]] : O.lid[B.perm[pos[best]]];
-        {
-            DropVals d;
-            if (STAGED) {
-                d.x1 = s_v[at]; d.x2 = s_v[kDepCap64 + at]; d.x3 = s_v[2 * kDepCap64 + at];
-                for (int a = 0; a < 3; ++a) {
-                    d.D[a] = s_v[(3 + a) * kDepCap64 + at];
-                    d.V[a] = s_v[(6 + a) * kDepCap64 + at];
-                }
-                d.T0 = s_v[9 * kDepCap64 + at]; d.H0 = s_v[10 * kDepCap64 + at];
-                d.E1 = s_v[11 * kDepCap64 + at]; d.E2 = s_v[12 * kDepCap64 + at];
-                d.mult = s_v[13 * kDepCap64 + at];
-            } else {
-                const int t = B.perm[at];
-                const DevPayload &P = B.pay;
-                d.x1 = O.x[0][t]; d.x2 = O.x[1][t]; d.x3 = O.x[2][t];
-                for (int a = 0; a < 3; ++a) { d.D[a] = P.D[a][t]; d.V[a] = P.V[a][t]; }
-                d.T0 = P.T0[t]; d.H0 = P.H0[t]; d.E1 = P.E1[t]; d.E2 = P.E2[t]; d.mult = P.mult[t];
+        if (pos[best] < end[best]) head[best] = O.lid[B.perm[pos[best]]];
+        DropVals d;
+        const int t = B.perm[at];
+        const DevPayload &P = B.pay;
+        d.x1 = O.x[0][t]; d.x2 = O.x[1][t]; d.x3 = O.x[2][t];
+        for (int a = 0; a < 3; ++a) { d.D[a] = P.D[a][t]; d.V[a] = P.V[a][t]; }
+        d.T0 = P.T0[t]; d.H0 = P.H0[t]; d.E1 = P.E1[t]; d.E2 = P.E2[t]; d.mult = P.mult[t];
+        contribute64(g, p, d, kpt, xv, yv, zv, acc);
+    }
+}
+
+// a / d, correctly rounded, from y = RN(1/d): two residual corrections.  The
+// first leaves a quotient within one ulp of a/d, and then the second returns
+// RN(a/d) (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990, theorem on q + r y with r = a - q d exact),
+// provided that d's significand is not all ones and nothing over- or
+// underflows: DevGrid::rdV is only set when the grid's denominators qualify,
+// and the caller has looked at the numerators.  5 operations for the
+// division's 14 instructions and its branch.
+__device__ __forceinline__ double div_by(double a, double d, double y) {
+    const double q0 = a * y;
+    const double q1 = fma(fma(-q0, d, a), y, q0);
+    return fma(fma(-q1, d, a), y, q1);
+}
+
+// numerators div_by may take: zero, or 2^-600 <= |v| < 2^900 (times weights
+// of at least 2^-159, their residuals stay normal numbers)
+__device__ __forceinline__ bool plain_num(double v) {
+    const unsigned hi = (unsigned)(__double_as_longlong(v) >> 32) & 0x7fffffffu;
+    return v == 0.0 || (hi >= ((1023u - 600u) << 20) && hi < ((1023u + 900u) << 20));
+}
+
+// stage of the FP64 tiles: droplet factors and trilinear weights, one array
+// of kDepCap64 per value
+enum { V64_D = 0, V64_V = 3, V64_T0 = 6, V64_H0, V64_E1, V64_E2, V64_MULT, V64_WX, V64_WY = V64_WX + 2,
+       V64_WZ = V64_WY + 2, V64_N = V64_WZ + 2 };
+
+// One node from the stage: its cells' lists (run[c]: first stage position, end
+// << 16; c = i<<2 | j<<1 | k) merged by lid.  dV, rdV: cell volume of the
+// droplet's cell and its reciprocal, for k = 0 and 1.
+template <bool FAST>
+__device__ __forceinline__ void merge_staged64(const DevParams &p, const int *s_lid, const double *s_v,
+                                               int (&run)[8], const double dV[2], const double rdV[2],
+                                               double acc[6]) {
+    constexpr int CAP = kDepCap64;
+    constexpr int kNone = 0x7fffffff;   // no lid is this large
+    int head[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) head[c] = (run[c] & 0xffff) < (run[c] >> 16) ? s_lid[run[c] & 0xffff] : kNone;
+    for (int q = 0; q < 6; ++q) acc[q] = 0.0;
+    while (true) {
+        int least = head[0];
+#pragma unroll
+        for (int c = 1; c < 8; ++c) least = min(least, head[c]);
+        if (least == kNone) break;
+        int o = 0, sel = 0;
+#pragma unroll
+        for (int c = 7; c >= 0; --c)
+            if (head[c] == least) { o = c; sel = run[c]; }
+        const int at = sel & 0xffff;
+        const int next = at + 1 < (sel >> 16) ? s_lid[at + 1] : kNone;
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+            if (c == o) { head[c] = next; run[c] = sel + 1; }
+        const double *v = s_v + at;
+        const double d = (o & 1) ? dV[1] : dV[0], y = (o & 1) ? rdV[1] : rdV[0];
+        const double wtx = v[(V64_WX + (o >> 2)) * CAP];
+        const double wty = v[(V64_WY + ((o >> 1) & 1)) * CAP];
+        const double wtz = v[(V64_WZ + (o & 1)) * CAP];
+        const double wtt = wtx * wty * wtz;
+        const double mult = v[V64_MULT * CAP];
+        auto term = [&](int q) {
+            const double a = v[q * CAP] * wtt;
+            return (FAST ? div_by(a, d, y) : a / d) * mult;
+        };
+        if (p.icouple == 1) {
+            for (int a = 0; a < 3; ++a) {
+                acc[a] = acc[a] - term(V64_D + a);
+                acc[a] = acc[a] - term(V64_V + a);
             }
-            contribute64(g, p, d, kpt, xv, yv, zv, acc);
+        }
+        if (p.iTcouple == 1) acc[3] = acc[3] - term(V64_T0);
+        if (p.iHcouple == 1) {
+            acc[4] = acc[4] - term(V64_H0);
+            acc[5] = acc[5] - term(V64_E1) + term(V64_E2);
         }
     }
 }
@@ -183,16 +247,11 @@ __device__ __forceinline__ void image_cells32(const DevBox &B, int px, int py, i
     }
 }
 
-// one pre-fold node image from global memory
-template <bool MIXED>
-__device__ __forceinline__ void image_global(const DevBox &B, const DevParams &p, int px, int py, int pz,
-                                             double acc[6]) {
-    if constexpr (MIXED) {
-        image_global32(B, p, px, py, pz, acc);
-        return;
-    }
+// FP64: one pre-fold node image from global memory
+__device__ __forceinline__ void image_global64(const DevBox &B, const DevParams &p, int px, int py, int pz,
+                                               double acc[6]) {
     const DevGrid &g = B.g;
-    int pos[8], end[8], ck[8], off[8];
+    int pos[8], end[8], ck[8];
     int n = 0;
     for (int i = 0; i <= 1; ++i)
         for (int j = 0; j <= 1; ++j)
@@ -201,9 +260,9 @@ __device__ __forceinline__ void image_global(const DevBox &B, const DevParams &p
                 if (ci < 1 || ci > g.nnx + 1 || cj < 1 || cj > g.nny + 1 || ckk < 0 || ckk > g.nnz) continue;
                 const int key = ckk + (g.nnz + 1) * ((cj - 1) + (g.nny + 1) * (ci - 1));
                 const int a = B.cell_start[key], b = B.cell_start[key + 1];
-                if (a < b) { pos[n] = a; end[n] = b; ck[n] = ckk; off[n] = (i << 2) | (j << 1) | k; n++; }
+                if (a < b) { pos[n] = a; end[n] = b; ck[n] = ckk; n++; }
             }
-    merge_ranges<false>(B, p, nullptr, nullptr, n, pos, end, ck, off, px, py, pz, acc);
+    merge_ranges(B, p, n, pos, end, ck, px, py, pz, acc);
 }
 
 // a whole output node (with its periodic images, folded x first, then y)
@@ -227,11 +286,15 @@ __device__ __forceinline__ void node_fold(const DevGrid &g, int ix, int iy, int 
     }
 }
 
-template <bool MIXED>
-__device__ __forceinline__ void node_global(const DevBox &B, const DevParams &p, int ix, int iy, int iz,
-                                            double out[6]) {
-    node_fold(B.g, ix, iy, iz, out,
-              [&](int px, int py, int pz, double acc[6]) { image_global<MIXED>(B, p, px, py, pz, acc); });
+// FP64: a node of a tile that does not stage, from global memory (out of line:
+// its locals stay off the staged path)
+__device__ __noinline__ void node_global64(const DevBox &B, const DevParams &p, int ix, int iy, int iz, bool images,
+                                           double out[6]) {
+    if (images)
+        image_global64(B, p, ix, iy, iz, out);
+    else
+        node_fold(B.g, ix, iy, iz, out,
+                  [&](int px, int py, int pz, double acc[6]) { image_global64(B, p, px, py, pz, acc); });
 }
 
 // Dense boxes (mixed): every cell's 8 corner sums S_o once, one thread per
@@ -269,9 +332,9 @@ __global__ void k_nodes_dense32(DevBox *boxes) {
     }
 }
 
-// a mixed deposition node: the box's own nodes to the sources, the
-// periodic images (mixed periodic boxes) to B.img
-__device__ __forceinline__ void store_node32(const DevBox &B, int ix, int iy, int iz, const double out[6]) {
+// a deposition node: the box's own nodes to the sources, the periodic images
+// (ix > nnx or iy > nny) to B.img
+__device__ __forceinline__ void store_node(const DevBox &B, int ix, int iy, int iz, const double out[6]) {
     const DevGrid &g = B.g;
     if (ix <= g.snx && iy <= g.sny) {
         const long long node = (long long)iz + (long long)g.nz2 * ((long long)(iy - 1) + (long long)g.sny * (ix - 1));
@@ -282,10 +345,10 @@ __device__ __forceinline__ void store_node32(const DevBox &B, int ix, int iy, in
     }
 }
 
-// Mixed periodic boxes: the fold of particle_coupling_exchange on the nodes
+// Periodic boxes: the fold of particle_coupling_exchange on the nodes
 // with ix <= 2 or iy <= 2, from their own image (in the sources) and the
 // image nodes, in node_fold's order; grid.y = box
-__global__ void k_fold32(DevBox *boxes) {
+__global__ void k_fold(DevBox *boxes) {
     const DevBox &B = boxes[blockIdx.y];
     const DevGrid &g = B.g;
     if (!g.periodic || B.img == nullptr || B.cellsum != nullptr) return;
@@ -323,31 +386,176 @@ __global__ void k_fold32(DevBox *boxes) {
 
 // shared memory of a tile shape (TX x TY x TZ nodes)
 __host__ __device__ constexpr int dep_smem_bytes(bool mixed, int TX, int TY, int TZ) {
-    return (mixed ? kDepCapMixed * 4 + kDepCapMixed * (kStageD * 8 + kStageF * 4) : kDepCap64 * 4 + 14 * kDepCap64 * 8) +
+    return (mixed ? kDepCapMixed * (kStageD * 8 + kStageF * 4) : kDepCap64 * (4 + V64_N * 8)) +
            (TX + 1) * (TY + 1) * (TZ + 2) * 4 + (TX + 1) * (TY + 1) * 4 + 16;
 }
 
-// Tiled deposition: tiles enumerate (z fastest) the node tiles of each box;
-// tile shapes 2x4x32, 4x4x16 and 2x2x64 nodes are instantiated (autotuned).
-template <bool MIXED, int kDepTX, int kDepTY, int kDepTZ>
-__global__ void __launch_bounds__(kDepositThreads, MIXED ? 4 : 2)
+// The columns of a tile's cells: s_cs[col][TZ+2] the starts of their cells in
+// the sorted list (absolute; levels z0-1 .. z0+TZ clamped to the grid),
+// s_off[col] their offsets in the stage.  Returns the droplets in all.
+template <int TX, int TY, int TZ>
+__device__ __forceinline__ int tile_columns(const DevBox &B, int x0, int y0, int z0, int *s_cs, int *s_off) {
+    constexpr int COLS = (TX + 1) * (TY + 1), CSW = TZ + 2;
+    static_assert(COLS <= 32, "one warp scans the column counts");
+    __shared__ int s_total;
+    const DevGrid &g = B.g;
+    const int ck_lo = max(z0 - 1, 0), ck_hi = min(z0 + TZ - 1, g.nnz);
+    for (int e = threadIdx.x; e < COLS * CSW; e += blockDim.x) {
+        const int cc = e / CSW, lzz = e % CSW;
+        const int ci = x0 - 1 + cc / (TY + 1), cj = y0 - 1 + cc % (TY + 1);
+        int v = 0;
+        if (ci >= 1 && cj >= 1 && ci <= g.nnx + 1 && cj <= g.nny + 1) {
+            const int ck = min(max(z0 - 1 + lzz, ck_lo), ck_hi + 1);
+            v = B.cell_start[ck + (g.nnz + 1) * ((cj - 1) + (g.nny + 1) * (ci - 1))];
+        }
+        s_cs[e] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        // exclusive scan of the columns' droplet counts (stage offsets)
+        const int cc = threadIdx.x;
+        const int cnt = cc < COLS ? s_cs[cc * CSW + CSW - 1] - s_cs[cc * CSW] : 0;
+        int incl = cnt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (cc >= o) incl += y;
+        }
+        if (cc < COLS) s_off[cc] = incl - cnt;
+        if (cc == COLS - 1) s_total = incl;
+    }
+    __syncthreads();
+    return s_total;
+}
+
+// FP64 tiles (z fastest); tile shapes 2x4x32, 4x4x16 and 2x2x64 nodes are
+// instantiated (autotuned).
+//
+// Bound by the FP64 pipe and the shared-memory pipe together: a node merges
+// about 8 droplets at one per cell, each of them 10 terms of a multiply, a
+// division, a multiply and a subtraction.  The trilinear weights (6 a droplet)
+// are formed while staging, not 3 per node, the divisions by the cell volume
+// take div_by, and the merge keeps its 8 list heads in registers.
+// 16.8 M droplets on 256^3: 8.00 -> 4.96 ms (FP64 pipe 24%, issue 43%: the
+// rest is the latency of the merge at 16 warps per SM); 1 M on 128^3: 0.71 ->
+// 0.49 ms, where the edge tiles' merges from global memory counted most.
+template <int TX, int TY, int TZ>
+__global__ void __launch_bounds__(kDepositThreads, 2)
+k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P) {
+    static_assert(TX * TY * TZ == kDepositThreads, "one thread per node of the tile");
+    constexpr int COLS = (TX + 1) * (TY + 1), CSW = TZ + 2, CAP = kDepCap64;
+    extern __shared__ __align__(16) unsigned char sm[];
+    double *s_v = (double *)sm;                    // [V64_N][CAP]
+    int *s_lid = (int *)(sm + V64_N * CAP * 8);    // [CAP]
+    int *s_cs = s_lid + CAP, *s_off = s_cs + COLS * CSW;
+    const Tile tl = tiles[blockIdx.x];
+    const DevBox &B = boxes[tl.box];
+    const DevGrid &g = B.g;
+    const int ntz = (g.nz2 + TZ - 1) / TZ, nty = (g.dny + TY - 1) / TY;
+    const int tzi = tl.start % ntz, tyi = (tl.start / ntz) % nty, txi = tl.start / (ntz * nty);
+    const int x0 = 1 + txi * TX, y0 = 1 + tyi * TY, z0 = tzi * TZ;
+    const int lz = threadIdx.x % TZ, ly = (threadIdx.x / TZ) % TY, lx = threadIdx.x / (TZ * TY);
+    const int ix = x0 + lx, iy = y0 + ly, iz = z0 + lz;
+    const bool valid = ix <= g.dnx && iy <= g.dny && iz <= g.nnz + 1;
+    // whether periodic images are nodes of their own (or there are none):
+    // otherwise the tiles on the periodic edges fold theirs from global memory
+    const bool images = !g.periodic || B.img != nullptr;
+    double out[6];
+    bool staged = images || ((x0 > 2) && (y0 > 2));
+    if (staged) {
+        const int total = tile_columns<TX, TY, TZ>(B, x0, y0, z0, s_cs, s_off);
+        staged = total <= CAP;
+        if (staged) {
+            // two droplets per pass: their loads are in flight together
+            const DevState &O = B.st[B.cur];
+            const DevPayload &Y = B.pay;
+            bool fast = g.rdV != nullptr;
+            auto stage = [&](int k, int c, const double *w, int l, int key) {
+                s_lid[k] = l;
+#pragma unroll
+                for (int q = 0; q < 11; ++q) s_v[q * CAP + k] = w[3 + q];
+#pragma unroll
+                for (int q = 0; q < 10; ++q) fast = fast && plain_num(w[3 + q]);
+                // the weights of the cell's lower (0) and upper (1) nodes
+                const int ci = x0 - 1 + c / (TY + 1), cj = y0 - 1 + c % (TY + 1);
+                const int ck = key - (g.nnz + 1) * ((cj - 1) + (g.nny + 1) * (ci - 1));
+                const double dz = g.dzu[ck + 1];
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    const double ax = fabs(w[0] - g.dx * (double)(ci + m + g.ioff - 1));
+                    const double ay = fabs(w[1] - g.dy * (double)(cj + m + g.joff - 1));
+                    const double az = fabs(w[2] - g.zz[ck + m]);
+                    const bool f = g.rdV != nullptr;
+                    s_v[(V64_WX + m) * CAP + k] = 1.0 - (f ? div_by(ax, g.dx, g.rdx) : ax / g.dx);
+                    s_v[(V64_WY + m) * CAP + k] = 1.0 - (f ? div_by(ay, g.dy, g.rdy) : ay / g.dy);
+                    s_v[(V64_WZ + m) * CAP + k] = 1.0 - (f ? div_by(az, dz, g.rdzu[ck + 1]) : az / dz);
+                }
+            };
+            for (int k0 = threadIdx.x; k0 < total; k0 += 2 * blockDim.x) {
+                const int k1 = k0 + blockDim.x;
+                const bool two = k1 < total;
+                int c0 = 0, c1 = 0;
+                while (c0 + 1 < COLS && s_off[c0 + 1] <= k0) ++c0;
+                while (c1 + 1 < COLS && s_off[c1 + 1] <= k1) ++c1;
+                const int t0 = B.perm[s_cs[c0 * CSW] + (k0 - s_off[c0])];
+                const int t1 = two ? B.perm[s_cs[c1 * CSW] + (k1 - s_off[c1])] : t0;
+                const double *src[14] = {O.x[0], O.x[1], O.x[2], Y.D[0], Y.D[1], Y.D[2], Y.V[0],
+                                         Y.V[1], Y.V[2], Y.T0, Y.H0, Y.E1, Y.E2, Y.mult};
+                double w0[14], w1[14];
+#pragma unroll
+                for (int q = 0; q < 14; ++q) {
+                    w0[q] = src[q][t0];
+                    w1[q] = src[q][t1];
+                }
+                const int l0 = O.lid[t0], l1 = O.lid[t1], e0 = B.key[t0], e1 = B.key[t1];
+                stage(k0, c0, w0, l0, e0);
+                if (two) stage(k1, c1, w1, l1, e1);
+            }
+            fast = __syncthreads_and(fast) != 0;
+            if (valid) {
+                int run[8];
+                double dV[2], rdV[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const int ck = iz - k;
+                    const bool in = ck >= 0 && ck <= g.nnz;
+                    dV[k] = in ? g.dx * g.dy * g.dzu[ck + 1] : 1.0;
+                    rdV[k] = in && g.rdV != nullptr ? g.rdV[ck + 1] : 1.0;
+#pragma unroll
+                    for (int ij = 0; ij < 4; ++ij) {
+                        const int cc = (lx + 1 - (ij >> 1)) * (TY + 1) + (ly + 1 - (ij & 1));
+                        const int *cs = s_cs + cc * CSW + lz + 1 - k;
+                        const int base = s_off[cc] - s_cs[cc * CSW];
+                        run[ij << 1 | k] = in ? (base + cs[0]) | (base + cs[1]) << 16 : 0;
+                    }
+                }
+                if (fast) merge_staged64<true>(P, s_lid, s_v, run, dV, rdV, out);
+                else merge_staged64<false>(P, s_lid, s_v, run, dV, rdV, out);
+            }
+        }
+    }
+    if (!valid) return;
+    if (!staged) node_global64(B, P, ix, iy, iz, images, out);
+    store_node(B, ix, iy, iz, out);
+}
+
+// Mixed tiles (z fastest), the same shapes.
+template <int kDepTX, int kDepTY, int kDepTZ>
+__global__ void __launch_bounds__(kDepositThreads, 4)
 k_deposit_tiled(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P, int *overflow_list,
                 int any_dense) {
     static_assert(kDepTX * kDepTY * kDepTZ == kDepositThreads, "one thread per node of the tile");
     constexpr int kDepCols = (kDepTX + 1) * (kDepTY + 1);
     constexpr int kDepCSW = kDepTZ + 2;
     extern __shared__ __align__(16) unsigned char sm[];
-    constexpr int CAP = MIXED ? kDepCapMixed : kDepCap64;
-    // stage: values first (8-byte aligned), then lid, cell starts, column offsets
-    double *s_v = (double *)sm;                                         // FP64: [14][CAP]; mixed: [kStageD][CAP]
-    float *s_f = (float *)(sm + kStageD * CAP * 8);                     // mixed: [kStageF][CAP]
-    int *s_lid = (int *)(sm + (MIXED ? CAP * (kStageD * 8 + kStageF * 4) : 14 * CAP * 8));
-    int *s_cs = s_lid + CAP;                                            // [cols][TZ+2], absolute
+    constexpr int CAP = kDepCapMixed;
+    // stage: values first (8-byte aligned), then cell starts, column offsets
+    double *s_v = (double *)sm;                                         // [kStageD][CAP]
+    float *s_f = (float *)(sm + kStageD * CAP * 8);                     // [kStageF][CAP]
+    int *s_cs = (int *)(sm + CAP * (kStageD * 8 + kStageF * 4));        // [cols][TZ+2], absolute
     int *s_off = s_cs + kDepCols * kDepCSW;                             // [cols] stage offset
-    __shared__ int s_total;
     const Tile tl = tiles[blockIdx.x];
     const DevBox &B = boxes[tl.box];
-    if (MIXED && any_dense && B.cellsum != nullptr) return;   // dense box: k_cellsums32 + k_nodes_dense32
+    if (any_dense && B.cellsum != nullptr) return;   // dense box: k_cellsums32 + k_nodes_dense32
     const DevParams &p = P;
     const DevGrid &g = B.g;
     const int ntz = (g.nz2 + kDepTZ - 1) / kDepTZ, nty = (g.dny + kDepTY - 1) / kDepTY;
@@ -356,181 +564,80 @@ k_deposit_tiled(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevPar
     const int lz = threadIdx.x % kDepTZ, ly = (threadIdx.x / kDepTZ) % kDepTY, lx = threadIdx.x / (kDepTZ * kDepTY);
     const int ix = x0 + lx, iy = y0 + ly, iz = z0 + lz;
     const bool valid = ix <= g.dnx && iy <= g.dny && iz <= g.nnz + 1;
-    const long long node = (long long)iz + (long long)g.nz2 * ((long long)(iy - 1) + (long long)g.sny * (ix - 1));
-    double out[6];
-    // FP64: tiles on the periodic edges merge from global memory with their
-    // images; mixed: every tile stages (images are nodes of their own)
-    bool staged = MIXED || ((x0 > 2) && (y0 > 2));
-    if (staged) {
-        const int ck_lo = max(z0 - 1, 0), ck_hi = min(z0 + kDepTZ - 1, g.nnz);
-        // cell starts of the tile's columns (absolute positions in the sorted list)
-        for (int e = threadIdx.x; e < kDepCols * kDepCSW; e += blockDim.x) {
-            const int cc = e / kDepCSW, lzz = e % kDepCSW;
-            const int ci = x0 - 1 + cc / (kDepTY + 1), cj = y0 - 1 + cc % (kDepTY + 1);
-            int v = 0;
-            if (ci >= 1 && cj >= 1 && ci <= g.nnx + 1 && cj <= g.nny + 1) {
-                const int ck = min(max(z0 - 1 + lzz, ck_lo), ck_hi + 1);
-                v = B.cell_start[ck + (g.nnz + 1) * ((cj - 1) + (g.nny + 1) * (ci - 1))];
-            }
-            s_cs[e] = v;
-        }
-        __syncthreads();
-        static_assert(kDepCols <= 32, "one warp scans the column counts");
-        if (threadIdx.x < 32) {
-            // exclusive scan of the columns' droplet counts (stage offsets)
-            const int cc = threadIdx.x;
-            const int cnt = cc < kDepCols ? s_cs[cc * kDepCSW + kDepCSW - 1] - s_cs[cc * kDepCSW] : 0;
-            int incl = cnt;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (cc >= o) incl += y;
-            }
-            if (cc < kDepCols) s_off[cc] = incl - cnt;
-            if (cc == kDepCols - 1) s_total = incl;
-        }
-        __syncthreads();
-        staged = s_total <= CAP;
-        if (staged) {
-            if (MIXED) {
-                // two droplets per pass: their perm and payload loads are in
-                // flight together
-                for (int k0 = threadIdx.x; k0 < s_total; k0 += 2 * blockDim.x) {
-                    const int k1 = k0 + blockDim.x;
-                    int c0 = 0, c1 = 0;
-                    while (c0 + 1 < kDepCols && s_off[c0 + 1] <= k0) ++c0;
-                    while (c1 + 1 < kDepCols && s_off[c1 + 1] <= k1) ++c1;
-                    const bool two = k1 < s_total;
-                    const int t0 = B.perm[s_cs[c0 * kDepCSW] + (k0 - s_off[c0])];
-                    const int t1 = two ? B.perm[s_cs[c1 * kDepCSW] + (k1 - s_off[c1])] : t0;
-                    float v0[P32_N], v1[P32_N];
-#pragma unroll
-                    for (int q = 0; q < P32_N; ++q) {
-                        v0[q] = B.pay32.f[q][t0];
-                        v1[q] = B.pay32.f[q][t1];
-                    }
-                    // the factors as contribute32 applies them: -DV, -T0, -H0, +E
-                    const double d0[kStageD] = {-(double)v0[P32_DV0], -(double)v0[P32_DV1], -(double)v0[P32_DV2],
-                                                -(double)v0[P32_T0], -(double)v0[P32_H0], (double)v0[P32_E]};
-                    const double d1[kStageD] = {-(double)v1[P32_DV0], -(double)v1[P32_DV1], -(double)v1[P32_DV2],
-                                                -(double)v1[P32_T0], -(double)v1[P32_H0], (double)v1[P32_E]};
-#pragma unroll
-                    for (int q = 0; q < kStageD; ++q) s_v[q * CAP + k0] = d0[q];
-                    s_f[0 * CAP + k0] = v0[P32_FX];
-                    s_f[1 * CAP + k0] = v0[P32_FY];
-                    s_f[2 * CAP + k0] = v0[P32_FZ];
-                    s_f[3 * CAP + k0] = v0[P32_FAC];
-                    if (two) {
-#pragma unroll
-                        for (int q = 0; q < kStageD; ++q) s_v[q * CAP + k1] = d1[q];
-                        s_f[0 * CAP + k1] = v1[P32_FX];
-                        s_f[1 * CAP + k1] = v1[P32_FY];
-                        s_f[2 * CAP + k1] = v1[P32_FZ];
-                        s_f[3 * CAP + k1] = v1[P32_FAC];
-                    }
-                }
-            }
-            if (!MIXED) {
-                // two droplets per pass, as for the mixed stage
-                const DevState &O = B.st[B.cur];
-                const DevPayload &P = B.pay;
-                for (int k0 = threadIdx.x; k0 < s_total; k0 += 2 * blockDim.x) {
-                    const int k1 = k0 + blockDim.x;
-                    const bool two = k1 < s_total;
-                    int c0 = 0, c1 = 0;
-                    while (c0 + 1 < kDepCols && s_off[c0 + 1] <= k0) ++c0;
-                    while (c1 + 1 < kDepCols && s_off[c1 + 1] <= k1) ++c1;
-                    const int t0 = B.perm[s_cs[c0 * kDepCSW] + (k0 - s_off[c0])];
-                    const int t1 = two ? B.perm[s_cs[c1 * kDepCSW] + (k1 - s_off[c1])] : t0;
-                    const double *src[14] = {O.x[0], O.x[1], O.x[2], P.D[0], P.D[1], P.D[2], P.V[0],
-                                             P.V[1], P.V[2], P.T0, P.H0, P.E1, P.E2, P.mult};
-                    double w0[14], w1[14];
-#pragma unroll
-                    for (int q = 0; q < 14; ++q) {
-                        w0[q] = src[q][t0];
-                        w1[q] = src[q][t1];
-                    }
-                    const int l0 = O.lid[t0], l1 = O.lid[t1];
-                    s_lid[k0] = l0;
-#pragma unroll
-                    for (int q = 0; q < 14; ++q) s_v[q * CAP + k0] = w0[q];
-                    if (two) {
-                        s_lid[k1] = l1;
-#pragma unroll
-                        for (int q = 0; q < 14; ++q) s_v[q * CAP + k1] = w1[q];
-                    }
-                }
-            }
-            __syncthreads();
-            if constexpr (MIXED) {
-              if (valid) {
-                for (int q = 0; q < 6; ++q) out[q] = 0.0;
-                // the corner loop stays rolled: a smaller kernel (instruction
-                // fetch was a leading stall)
-#pragma unroll 1
-                for (int o = 0; o < 8; ++o) {
-                    const int i = o >> 2, j = (o >> 1) & 1, k = o & 1;
-                    const int ckk = iz - k;
-                    if (ckk < 0 || ckk > g.nnz) continue;
-                    const int cc = (lx + 1 - i) * (kDepTY + 1) + (ly + 1 - j);
-                    const int lzz = lz + 1 - k;
-                    const int base = s_off[cc] - s_cs[cc * kDepCSW];
-                    const int a = base + s_cs[cc * kDepCSW + lzz];
-                    const int b = base + s_cs[cc * kDepCSW + lzz + 1];
-                    if (a == b) continue;
-                    double S[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-                    for (int at = a; at < b; ++at) {
-                        // contribute32 with the factors staged in FP64 (the
-                        // same values, so the same bits)
-                        const float fx = s_f[at], fy = s_f[CAP + at], fz = s_f[2 * CAP + at];
-                        const float wx = i ? fx : 1.0f - fx;
-                        const float wy = j ? fy : 1.0f - fy;
-                        const float wz = k ? fz : 1.0f - fz;
-                        const double c = (double)(wx * wy * wz * s_f[3 * CAP + at]);
-                        if (p.icouple == 1)
-                            for (int a3 = 0; a3 < 3; ++a3) S[a3] = fma(s_v[a3 * CAP + at], c, S[a3]);
-                        if (p.iTcouple == 1) S[3] = fma(s_v[3 * CAP + at], c, S[3]);
-                        if (p.iHcouple == 1) {
-                            S[4] = fma(s_v[4 * CAP + at], c, S[4]);
-                            S[5] = fma(s_v[5 * CAP + at], c, S[5]);
-                        }
-                    }
-                    for (int q = 0; q < 6; ++q) out[q] += S[q];
-                }
-              }
-            } else if (valid) {
-                int pos[8], end[8], ck[8], off[8];
-                int n = 0;
-                for (int i = 0; i <= 1; ++i)
-                    for (int j = 0; j <= 1; ++j)
-                        for (int k = 0; k <= 1; ++k) {
-                            const int ckk = iz - k;
-                            if (ckk < 0 || ckk > g.nnz) continue;
-                            const int cc = (lx + 1 - i) * (kDepTY + 1) + (ly + 1 - j);
-                            const int lzz = lz + 1 - k;
-                            const int base = s_off[cc] - s_cs[cc * kDepCSW];
-                            const int a = base + s_cs[cc * kDepCSW + lzz];
-                            const int b = base + s_cs[cc * kDepCSW + lzz + 1];
-                            if (a < b) {
-                                pos[n] = a; end[n] = b; ck[n] = ckk; off[n] = (i << 2) | (j << 1) | k; n++;
-                            }
-                        }
-                merge_ranges<true>(B, p, s_lid, s_v, n, pos, end, ck, off, ix, iy, iz, out);
-            }
-        }
-    }
-    if (MIXED) {
-        if (!staged) {
-            // above the stage capacity: k_deposit_overflow32, which has the
-            // registers of the global path
-            if (threadIdx.x == 0) overflow_list[1 + atomicAdd(overflow_list, 1)] = blockIdx.x;
-            return;
-        }
-        if (valid) store_node32(B, ix, iy, iz, out);
+    const int total = tile_columns<kDepTX, kDepTY, kDepTZ>(B, x0, y0, z0, s_cs, s_off);
+    if (total > CAP) {
+        // above the stage capacity: k_deposit_overflow32, which has the
+        // registers of the global path
+        if (threadIdx.x == 0) overflow_list[1 + atomicAdd(overflow_list, 1)] = blockIdx.x;
         return;
     }
-    if (!staged && valid) node_global<MIXED>(B, p, ix, iy, iz, out);
-    if (valid)
-        for (int q = 0; q < 6; ++q) B.src[q][node] = out[q];
+    // two droplets per pass: their perm and payload loads are in flight
+    // together
+    for (int k0 = threadIdx.x; k0 < total; k0 += 2 * blockDim.x) {
+        const int k1 = k0 + blockDim.x;
+        int c0 = 0, c1 = 0;
+        while (c0 + 1 < kDepCols && s_off[c0 + 1] <= k0) ++c0;
+        while (c1 + 1 < kDepCols && s_off[c1 + 1] <= k1) ++c1;
+        const bool two = k1 < total;
+        const int t0 = B.perm[s_cs[c0 * kDepCSW] + (k0 - s_off[c0])];
+        const int t1 = two ? B.perm[s_cs[c1 * kDepCSW] + (k1 - s_off[c1])] : t0;
+        float v0[P32_N], v1[P32_N];
+#pragma unroll
+        for (int q = 0; q < P32_N; ++q) {
+            v0[q] = B.pay32.f[q][t0];
+            v1[q] = B.pay32.f[q][t1];
+        }
+        // the factors as contribute32 applies them: -DV, -T0, -H0, +E
+        auto stage = [&](int k, const float *v) {
+            const double d[kStageD] = {-(double)v[P32_DV0], -(double)v[P32_DV1], -(double)v[P32_DV2],
+                                       -(double)v[P32_T0], -(double)v[P32_H0], (double)v[P32_E]};
+#pragma unroll
+            for (int q = 0; q < kStageD; ++q) s_v[q * CAP + k] = d[q];
+            s_f[0 * CAP + k] = v[P32_FX];
+            s_f[1 * CAP + k] = v[P32_FY];
+            s_f[2 * CAP + k] = v[P32_FZ];
+            s_f[3 * CAP + k] = v[P32_FAC];
+        };
+        stage(k0, v0);
+        if (two) stage(k1, v1);
+    }
+    __syncthreads();
+    if (!valid) return;
+    double out[6];
+    for (int q = 0; q < 6; ++q) out[q] = 0.0;
+    // the corner loop stays rolled: a smaller kernel (instruction fetch was a
+    // leading stall)
+#pragma unroll 1
+    for (int o = 0; o < 8; ++o) {
+        const int i = o >> 2, j = (o >> 1) & 1, k = o & 1;
+        const int ckk = iz - k;
+        if (ckk < 0 || ckk > g.nnz) continue;
+        const int cc = (lx + 1 - i) * (kDepTY + 1) + (ly + 1 - j);
+        const int lzz = lz + 1 - k;
+        const int base = s_off[cc] - s_cs[cc * kDepCSW];
+        const int a = base + s_cs[cc * kDepCSW + lzz];
+        const int b = base + s_cs[cc * kDepCSW + lzz + 1];
+        if (a == b) continue;
+        double S[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        for (int at = a; at < b; ++at) {
+            // contribute32 with the factors staged in FP64 (the same values,
+            // so the same bits)
+            const float fx = s_f[at], fy = s_f[CAP + at], fz = s_f[2 * CAP + at];
+            const float wx = i ? fx : 1.0f - fx;
+            const float wy = j ? fy : 1.0f - fy;
+            const float wz = k ? fz : 1.0f - fz;
+            const double c = (double)(wx * wy * wz * s_f[3 * CAP + at]);
+            if (p.icouple == 1)
+                for (int a3 = 0; a3 < 3; ++a3) S[a3] = fma(s_v[a3 * CAP + at], c, S[a3]);
+            if (p.iTcouple == 1) S[3] = fma(s_v[3 * CAP + at], c, S[3]);
+            if (p.iHcouple == 1) {
+                S[4] = fma(s_v[4 * CAP + at], c, S[4]);
+                S[5] = fma(s_v[5 * CAP + at], c, S[5]);
+            }
+        }
+        for (int q = 0; q < 6; ++q) out[q] += S[q];
+    }
+    store_node(B, ix, iy, iz, out);
 }
 
 // Mixed tiles listed by k_deposit_tiled (overflow_list[0] of them in
@@ -552,7 +659,7 @@ k_deposit_overflow32(DevBox *boxes, const Tile *tiles, const __grid_constant__ D
         if (ix > g.dnx || iy > g.dny || iz > g.nnz + 1) continue;
         double out[6];
         image_global32(B, P, ix, iy, iz, out);
-        store_node32(B, ix, iy, iz, out);
+        store_node(B, ix, iy, iz, out);
     }
 }
 

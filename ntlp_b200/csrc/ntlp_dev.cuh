@@ -39,6 +39,10 @@ struct DevGrid {
     double dx, dy, xl, yl, zl;
     double rdx, rdy;       // 1/dx, 1/dy
     const double *z, *zz, *dzw, *dzu;
+    // FP64 deposition: 1/dzu(k) and 1/(dx dy dzu(k)), correctly rounded, like
+    // rdx and rdy; NULL when one of the denominators does not qualify for the
+    // division by reciprocal (see div_by)
+    const double *rdzu, *rdV;
     long long ncells;      // (nnx+1)(nny+1)(nnz+1)
     long long nnodes;      // (nnz+2)*nny*nnx
     // Bucket tables that start the level searches (NULL: plain binary
@@ -60,9 +64,9 @@ struct DevGrid {
     int periodic;
     int ioff, joff;
     int snx, sny;
-    // node extents of the deposition tiles: snx, sny, and for mixed
-    // periodic boxes 2 more (the periodic images, deposited as nodes and
-    // folded in afterwards)
+    // node extents of the deposition tiles: snx, sny, and for periodic
+    // boxes with an image buffer 2 more (the periodic images, deposited as
+    // nodes and folded in afterwards)
     int dnx, dny;
     double xmin, xmax, ymin, ymax;   // set_bounds (particles.f90:1766-1781)
 };
@@ -167,7 +171,7 @@ struct DevBox {
     double *src[6];        // [nnodes] each, column layout
     int *err;              // device error word (0 = fine)
     int *big_cells;        // this sort has cells of more than kSmallCell droplets
-    double *img;           // mixed periodic boxes: [6][img_count] image nodes (ix > nnx or iy > nny)
+    double *img;           // periodic boxes: [6][img_count] image nodes (ix > nnx or iy > nny)
     double *cellsum;       // mixed boxes with many droplets per cell: [ncells][8 corners][6]
                            // per-cell source sums (nullptr: tiled deposition)
     int *defer;            // [cap] droplets whose Gauss-Newton solve failed this step
@@ -257,7 +261,7 @@ __device__ __forceinline__ long long ext_index(const DevGrid &g, int k, int j, i
 
 __device__ __forceinline__ double cube(double r) { return (r * r) * r; }
 
-// image nodes of a mixed periodic box (its deposition nodes with ix > nnx,
+// image nodes of a periodic box (its deposition nodes with ix > nnx,
 // iy in 1..nny+2, then those with iy > nny, ix in 1..nnx), per quantity
 __host__ __device__ __forceinline__ long long img_count(const DevGrid &g) {
     return (long long)(2 * (g.nny + 2) + 2 * g.nnx) * g.nz2;

@@ -465,14 +465,14 @@ void launch_payload64(DevBox *boxes, const Tile *tiles, int ntiles, const DevPar
 template <int V>
 static void dep64(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P, cudaStream_t st) {
     constexpr int TX = kDepShape[V][0], TY = kDepShape[V][1], TZ = kDepShape[V][2];
-    k_deposit_tiled<false, TX, TY, TZ>
-        <<<ntiles, kDepositThreads, dep_smem_bytes(false, TX, TY, TZ), st>>>(boxes, tiles, P, nullptr, 0);
+    k_deposit64<TX, TY, TZ>
+        <<<ntiles, kDepositThreads, dep_smem_bytes(false, TX, TY, TZ), st>>>(boxes, tiles, P);
 }
 
 template <int V>
 static void dep64_attr() {
     constexpr int TX = kDepShape[V][0], TY = kDepShape[V][1], TZ = kDepShape[V][2];
-    cudaFuncSetAttribute(k_deposit_tiled<false, TX, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_deposit64<TX, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          dep_smem_bytes(false, TX, TY, TZ));
 }
 
@@ -484,12 +484,13 @@ void prepare_kernels64() {
 }
 
 void launch_deposit64(int variant, DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P,
-                      cudaStream_t st) {
+                      cudaStream_t st, int nbox) {
     if (ntiles <= 0) return;
     prepare_kernels64();
     if (variant == 1) dep64<1>(boxes, tiles, ntiles, P, st);
     else if (variant == 2) dep64<2>(boxes, tiles, ntiles, P, st);
     else dep64<0>(boxes, tiles, ntiles, P, st);
+    if (nbox > 0) k_fold<<<dim3(kFoldBlocks, nbox), 256, 0, st>>>(boxes);
 }
 
 }  // namespace ntlp

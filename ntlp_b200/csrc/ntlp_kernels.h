@@ -42,8 +42,10 @@ void launch_update_rk3_64(int ilin, DevBox *boxes, const Tile *tiles, int ntiles
                           StepIn in, cudaStream_t st);
 void launch_payload64(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P, double dt,
                       cudaStream_t st);
+// nbox: boxes whose periodic images are deposited as nodes, to be folded in (0:
+// none, the tiles on the periodic edges fold their own)
 void launch_deposit64(int variant, DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P,
-                      cudaStream_t st);
+                      cudaStream_t st, int nbox);
 
 // mixed precision (ntlp_mixed.cu)
 // blk_kb > 0 (6th order): the interpolation runs over cell blocks of
@@ -79,7 +81,7 @@ void launch_deposit_mixed(int variant, DevBox *boxes, const Tile *tiles, int nti
                           cudaStream_t st, int nbox, bool dense, int *overflow_list);
 constexpr int kDenseRatio = 16;     // mixed boxes with capacity >= 16 x cells use per-cell sums
 constexpr int kDenseBlocks = 1184;  // grid.x of the cell-sum kernels
-constexpr int kFoldBlocks = 148;    // grid.x of the periodic fold (mixed)
+constexpr int kFoldBlocks = 148;    // grid.x of the periodic fold
 // kernel attributes (dynamic shared memory of the deposition), set once per
 // device, on the device that is current; call outside stream capture
 void prepare_kernels64();

@@ -654,7 +654,7 @@ static void depm(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &
                  int *overflow_list, bool dense) {
     constexpr int TX = kDepShape[V][0], TY = kDepShape[V][1], TZ = kDepShape[V][2];
     cudaMemsetAsync(overflow_list, 0, sizeof(int), st);
-    k_deposit_tiled<true, TX, TY, TZ>
+    k_deposit_tiled<TX, TY, TZ>
         <<<ntiles, kDepositThreads, dep_smem_bytes(true, TX, TY, TZ), st>>>(boxes, tiles, P, overflow_list,
                                                                            dense ? 1 : 0);
     const int g = ntiles < kDenseBlocks ? ntiles : kDenseBlocks;
@@ -664,7 +664,7 @@ static void depm(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &
 template <int V>
 static void depm_attr() {
     constexpr int TX = kDepShape[V][0], TY = kDepShape[V][1], TZ = kDepShape[V][2];
-    cudaFuncSetAttribute(k_deposit_tiled<true, TX, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_deposit_tiled<TX, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          dep_smem_bytes(true, TX, TY, TZ));
 }
 
@@ -682,7 +682,7 @@ void launch_deposit_mixed(int variant, DevBox *boxes, const Tile *tiles, int nti
     if (variant == 1) depm<1>(boxes, tiles, ntiles, P, st, overflow_list, dense);
     else if (variant == 2) depm<2>(boxes, tiles, ntiles, P, st, overflow_list, dense);
     else depm<0>(boxes, tiles, ntiles, P, st, overflow_list, dense);
-    k_fold32<<<dim3(kFoldBlocks, nbox), 256, 0, st>>>(boxes);
+    k_fold<<<dim3(kFoldBlocks, nbox), 256, 0, st>>>(boxes);
     if (dense) {
         k_cellsums32<<<dim3(kDenseBlocks, nbox), 256, 0, st>>>(boxes, P);
         k_nodes_dense32<<<dim3(kDenseBlocks, nbox), 256, 0, st>>>(boxes);

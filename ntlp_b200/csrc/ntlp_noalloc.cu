@@ -248,7 +248,7 @@ extern "C" int ntlp_coupling_noalloc(const ntlp_grid *grid, const ntlp_params *p
     launch_sort(B_d, plan, st);
     launch_finish(B_d, 1, st);
     launch_payload64(B_d, drop_tiles, nd, dp, dt, st);
-    launch_deposit64(0, B_d, node_tiles, nn, dp, st);
+    launch_deposit64(0, B_d, node_tiles, nn, dp, st, 0);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         fprintf(stderr, "ntlp_coupling_noalloc: %s\n", cudaGetErrorString(e));
