@@ -142,7 +142,6 @@ struct ntlp_ctx {
     Tile *blk_tiles_d = nullptr;
     int n_blk_tiles = 0;
     int blk_tile_cap = 0;   // tiles blk_tiles_d holds (the smallest block height the tuner tries)
-    bool tex_all64 = true;   // every box's FP64 fields have textures (FP64)
     bool any_dense = false;   // some box deposits through per-cell sums (mixed)
     int64_t g_launches = 0;
     int64_t bytes = 0;
@@ -203,27 +202,6 @@ unsigned long long f4_texture(const float4 *base, size_t count) {
     rd.res.linear.devPtr = (void *)base;
     rd.res.linear.desc = cudaCreateChannelDesc<float4>();
     rd.res.linear.sizeInBytes = count * sizeof(float4);
-    cudaTextureDesc td{};
-    td.addressMode[0] = cudaAddressModeClamp;
-    td.filterMode = cudaFilterModePoint;
-    td.readMode = cudaReadModeElementType;
-    td.normalizedCoords = 0;
-    cudaTextureObject_t t = 0;
-    if (cudaCreateTextureObject(&t, &rd, &td, nullptr) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return (unsigned long long)t;
-}
-
-// an FP64 field (count elements) as a 1D linear texture of int2, read
-// element by element; 0 when the device refuses it
-unsigned long long f64_texture(const double *base, size_t count) {
-    cudaResourceDesc rd{};
-    rd.resType = cudaResourceTypeLinear;
-    rd.res.linear.devPtr = (void *)base;
-    rd.res.linear.desc = cudaCreateChannelDesc<int2>();
-    rd.res.linear.sizeInBytes = count * sizeof(double);
     cudaTextureDesc td{};
     td.addressMode[0] = cudaAddressModeClamp;
     td.filterMode = cudaFilterModePoint;
@@ -309,12 +287,14 @@ void carve_box(Carver &cv, BoxHost &h, DevBox &B, bool mixed) {
         B.g.lut_zz = lut; B.g.lut_z = lut + kLutPerLevel * g.nz2;
         B.g.rden_zz = rden; B.g.rden_z = rden + 6 * (g.nnz + 3);
     }
-    for (int k = 0; k < 5; ++k) {
-        double *f;
-        // FP64 path: + 1 KB, to start the texture on a 1 KB boundary
-        cv.take(&f, npad + (mixed ? 0 : 128));
-        if (f && !mixed) f = (double *)(((uintptr_t)f + 1023) & ~(uintptr_t)1023);
-        B.f[k] = f;
+    B.f64 = nullptr; B.fw64 = nullptr; B.f4 = nullptr; B.fw = nullptr; B.ref = nullptr;
+    if (!mixed) {
+        Node64 *f;
+        double *w;
+        cv.take(&f, npad);
+        cv.take(&w, npad);
+        B.f64 = f;
+        B.fw64 = w;
     }
     if (mixed) {
         // guard elements on both sides: the 6-level window loads of the
@@ -322,12 +302,15 @@ void carve_box(Carver &cv, BoxHost &h, DevBox &B, bool mixed) {
         // after the last (with zero weight); the guards keep them in bounds
         float4 *f4;
         float *fw;
+        double *ref;
         // + 1 KB, to start the texture on a 1 KB boundary (the device's
         // texture alignment is smaller)
         cv.take(&f4, npad + 2 * kF32Guard + 64);
         if (f4) f4 = (float4 *)(((uintptr_t)f4 + 1023) & ~(uintptr_t)1023);
         cv.take(&fw, npad + 2 * kF32Guard);
+        cv.take(&ref, 5);
         if (cv.base) {
+            B.ref = ref;
             B.f4 = f4 + kF32Guard;
             B.fw = fw + kF32Guard;
         }
@@ -379,6 +362,7 @@ void carve_box(Carver &cv, BoxHost &h, DevBox &B, bool mixed) {
     const size_t halo = 6 * (size_t)g.nz2 * (size_t)(g.snx > g.sny ? g.snx : g.sny);
     if (halo > stage) stage = halo;
     if (flow_n > stage) stage = flow_n;
+    if (npad > stage) stage = npad;
     if (tiles > stage) stage = tiles;
     cv.take(&h.staging, stage);
     cv.take(&h.rank, n);
@@ -627,8 +611,6 @@ extern "C" void ntlp_ctx_destroy(ntlp_ctx *c) {
     for (cudaEvent_t e : c->tev) cudaEventDestroy(e);
     for (const DevBox &B : c->box) {
         if (B.tex_f4) cudaDestroyTextureObject((cudaTextureObject_t)B.tex_f4);
-        for (int q = 0; q < 5; ++q)
-            if (B.tex_f64[q]) cudaDestroyTextureObject((cudaTextureObject_t)B.tex_f64[q]);
     }
     for (auto &h : c->bh) {
         if (h.arena) cudaFreeAsync(h.arena, c->stream);
@@ -800,18 +782,14 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
         if (mixed) {
             const size_t npad = (size_t)nz2 * B.g.ny5 * B.g.nx5 + 2 * kF32Guard;
             if (cudaMemsetAsync((void *)(B.f4 - kF32Guard), 0, npad * sizeof(float4), c->stream) ||
-                cudaMemsetAsync((void *)(B.fw - kF32Guard), 0, npad * sizeof(float), c->stream))
+                cudaMemsetAsync((void *)(B.fw - kF32Guard), 0, npad * sizeof(float), c->stream) ||
+                cudaMemsetAsync((void *)B.ref, 0, 5 * sizeof(double), c->stream))
                 return bail(fail(c, NTLP_ERR_CUDA, "initialising box %d failed", b));
-            for (int q = 0; q < 5; ++q) B.tex_f64[q] = 0;
             B.tex_f4 = f4_texture(B.f4 - kF32Guard, npad);
             if (!B.tex_f4) c->tex_all = false;
             if (B.cellsum) c->any_dense = true;
         } else {
             B.tex_f4 = 0;
-            for (int q = 0; q < 5; ++q) {
-                B.tex_f64[q] = f64_texture(B.f[q], (size_t)nz2 * B.g.ny5 * B.g.nx5);
-                if (!B.tex_f64[q]) c->tex_all64 = false;
-            }
         }
         if (cudaMemcpyAsync((void *)B.g.lut_zz, h.lut.data(), h.lut.size() * sizeof(int), cudaMemcpyHostToDevice,
                             c->stream) ||
@@ -958,35 +936,32 @@ int alloc_rk3(ntlp_ctx *c) {
     return push_boxes(c);
 }
 
-int fields_ext(ntlp_ctx *c, int b, const double *const h[5]) {
+// The box's stored fields from the caller's five arrays (flow or halo-padded
+// layout).  Arrays in this device's memory are read where they are, in one
+// launch; the others pass through the staging buffer one by one.
+int fields_in(ntlp_ctx *c, int b, const double *const h[5], bool flow) {
     if (!box_ok(c, b)) return fail(c, NTLP_ERR_ARG, "box %d out of range", b);
-    for (int k = 0; k < 5; ++k)
-        if (!h[k]) return fail(c, NTLP_ERR_ARG, "field %d is NULL", k);
-    const DevBox &B = c->box[b];
-    const size_t npad = (size_t)B.g.nz2 * B.g.ny5 * B.g.nx5;
-    for (int k = 0; k < 5; ++k)
-        CK(cudaMemcpyAsync((void *)B.f[k], h[k], npad * 8, cudaMemcpyDefault, c->stream));
-    if (B.f4) launch_pack_f32(&B, (float4 *)B.f4, (float *)B.fw, c->stream);
-    CK(cudaGetLastError());
-    c->bh[b].have_fields = true;
-    if (b == 0) c->up_pending = false;
-    return NTLP_OK;
-}
-
-int fields_flow(ntlp_ctx *c, int b, const double *const h[5]) {
-    if (!box_ok(c, b)) return fail(c, NTLP_ERR_ARG, "box %d out of range", b);
-    if (!c->box[b].g.periodic)
+    if (flow && !c->box[b].g.periodic)
         return fail(c, NTLP_ERR_STATE, "a subdomain takes its fields with halos (ntlp_fields_upload_ext)");
     for (int k = 0; k < 5; ++k)
         if (!h[k]) return fail(c, NTLP_ERR_ARG, "field %d is NULL", k);
     const DevBox &B = c->box[b];
-    const size_t nflow = (size_t)B.g.nnx * B.g.nny * B.g.nz2;
-    double *stg = c->bh[b].staging;
+    const DevGrid &g = B.g;
+    const size_t n = flow ? (size_t)g.nnx * g.nny * g.nz2 : (size_t)g.nz2 * g.ny5 * g.nx5;
+    FieldSrc here{};
+    bool any = false;
     for (int k = 0; k < 5; ++k) {
-        CK(cudaMemcpyAsync(stg, h[k], nflow * 8, cudaMemcpyDefault, c->stream));
-        launch_fill_ext(stg, (double *)B.f[k], B.g, c->stream);
+        if (on_device(c, h[k], 8)) {
+            here.p[k] = h[k];
+            any = true;
+            continue;
+        }
+        FieldSrc one{};
+        one.p[k] = c->bh[b].staging;
+        CK(cudaMemcpyAsync(c->bh[b].staging, h[k], n * 8, cudaMemcpyDefault, c->stream));
+        launch_fill_fields(B, one, flow, c->stream);
     }
-    if (B.f4) launch_pack_f32(&B, (float4 *)B.f4, (float *)B.fw, c->stream);
+    if (any) launch_fill_fields(B, here, flow, c->stream);
     CK(cudaGetLastError());
     c->bh[b].have_fields = true;
     if (b == 0) c->up_pending = false;
@@ -1061,11 +1036,12 @@ int consume_upload(ntlp_ctx *c) {
     const size_t nflow = (size_t)B.g.nnx * B.g.nny * B.g.nz2;
     const int a = c->up_cur;
     CK(cudaStreamWaitEvent(c->stream, c->ev_up[a], 0));
-    for (int k = 0; k < 5; ++k) launch_fill_ext(c->up_area[a] + k * nflow, (double *)B.f[k], B.g, c->stream);
-    if (B.f4) launch_pack_f32(&B, (float4 *)B.f4, (float *)B.fw, c->stream);
+    FieldSrc src;
+    for (int k = 0; k < 5; ++k) src.p[k] = c->up_area[a] + k * nflow;
+    launch_fill_fields(B, src, true, c->stream);
     CK(cudaGetLastError());
     CK(cudaEventRecord(c->ev_fill[a], c->stream));
-    c->launches += B.f4 ? 6 : 5;
+    c->launches += 1;
     c->fill_recorded[a] = true;
     c->up_pending = false;
     return NTLP_OK;
@@ -1235,12 +1211,12 @@ int launch_step(ntlp_ctx *c, int kind, int istage, double dt, int32_t it, bool w
                                    c->n_blk_tiles);
         else
             launch_update_be64(c->params.ilin, nt, c->box_d, c->drop_tiles_d[c->nt_variant],
-                               c->n_drop_tiles[c->nt_variant], c->nbox, c->dp, in, c->stream, c->tex_all64);
+                               c->n_drop_tiles[c->nt_variant], c->nbox, c->dp, in, c->stream);
         c->launches += kUpdateLaunches;
     } else {
         launch_update_rk3_64(c->params.ilin, c->box_d, c->drop_tiles_d[0], c->n_drop_tiles[0], c->dp, in,
                              c->stream);
-        c->launches += 1;
+        c->launches += 2;   // interpolation, stage
     }
     phase_end(c, PH_UPDATE, e0);
     e0 = phase_begin(c);
@@ -1610,7 +1586,7 @@ int ntlp_box_fields_upload_ext(ntlp_ctx *c, int32_t box, const double *uext, con
                                const double *Text, const double *T2ext) {
     if (!c) return NTLP_ERR_ARG;
     const double *h[5] = {uext, vext, wext, Text, T2ext};
-    return fields_ext(c, box, h);
+    return fields_in(c, box, h, false);
 }
 
 int ntlp_fields_upload(ntlp_ctx *c, const double *u, const double *v, const double *w, const double *t,
@@ -1622,7 +1598,7 @@ int ntlp_box_fields_upload(ntlp_ctx *c, int32_t box, const double *u, const doub
                            const double *t, const double *q) {
     if (!c) return NTLP_ERR_ARG;
     const double *h[5] = {u, v, w, t, q};
-    return fields_flow(c, box, h);
+    return fields_in(c, box, h, true);
 }
 
 int ntlp_droplets_upload(ntlp_ctx *c, const ntlp_droplets *d) { return ntlp_box_droplets_upload(c, 0, d); }

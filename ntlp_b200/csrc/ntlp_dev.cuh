@@ -1,9 +1,11 @@
 // ntlp_dev.cuh -- device-side descriptors and helpers of the droplet step.
 //
 // Layout in HBM (one "box" = one periodic domain with its own grid):
-//   fields  f(0:nnz+1, -1:nny+3, -1:nnx+3), z fastest, FP64 (and an FP32
-//           copy for the mixed path): the reference's uext layout
-//           (particles.f90:5-10).
+//   fields  f(0:nnz+1, -1:nny+3, -1:nnx+3), z fastest: the reference's uext
+//           index order (particles.f90:5-10), stored as the interpolation
+//           reads them: (u, v, T, q) packed per point and w apart, since it
+//           has its own vertical levels; FP64 (FP64 path) or FP32 deviations
+//           (mixed path).
 //   droplets structure of arrays, two buffers (A/B).  A step reads buffer
 //           `cur` through the permutation `perm` (cell-sorted order) and
 //           writes buffer 1-cur in that order, so the permutation costs no
@@ -138,6 +140,11 @@ constexpr int kBlkWinX = kBlkX + 5, kBlkWinY = kBlkY + 5;
 // bits of the device error word (DevBox::err)
 enum { ERR_STAGE_WAIT = 1 };   // a staged tile did not arrive within the wait limit
 
+// the FP64 fields of a point that share its vertical levels: one 32-byte load
+struct alignas(32) Node64 {
+    double u, v, T, q;
+};
+
 struct DevBox {
     // TMA descriptor (CUtensorMap, 128 bytes) of the packed (u, v, T, q)
     // FP32 copy f4, viewed as floats (4*nz2, ny5, nx5), box (4*(kb+8), 9, 9);
@@ -145,15 +152,14 @@ struct DevBox {
     alignas(64) unsigned char tmap_f4[128];
     int blk_kb;            // z cells per interpolation block; 0: no staged interpolation
     DevGrid g;
-    const double *f[5];    // u v w T q, halo-padded FP64
+    const Node64 *f64;     // FP64 path: (u, v, T, q) packed per point
+    const double *fw64;    // FP64 path: w
+    const double *ref;     // mixed path: the five fields' reference values (u, v, w, T, q)
     const float4 *f4;      // mixed path: (u, v, T, q) deviations packed per point
     const float *fw;       // mixed path: w deviation
     // mixed path: f4 as a 1D linear texture (element 0 = the first guard
     // element, f4 - kF32GuardDev), 0 when the device refused it
     unsigned long long tex_f4;
-    // FP64 path: the five FP64 fields as 1D linear textures of int2 (the
-    // same 8 bytes per element), 0 when the device refused them
-    unsigned long long tex_f64[5];
     DevState st[2];
     DevPayload pay;
     DevPayload32 pay32;    // mixed path
@@ -273,7 +279,8 @@ __host__ __device__ __forceinline__ long long img_index(const DevGrid &g, int ix
 
 // The FP32 field copies hold deviations from the value at the interior
 // point (k, j, i) = (1, 1, 1): T ~ 293 K would otherwise keep only ~3e-5 K
-// in FP32, and the saturation vapour pressure is exponential in T.
+// in FP32, and the saturation vapour pressure is exponential in T.  DevBox::ref
+// keeps the values.
 __host__ __device__ __forceinline__ long long f32_ref_index(const DevGrid &g) {
     return 1LL + (long long)g.nz2 * (2LL + (long long)g.ny5 * 2LL);
 }

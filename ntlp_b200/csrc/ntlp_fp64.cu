@@ -21,6 +21,13 @@ namespace ntlp {
 // ---------------------------------------------------------------------------
 // interpolation (particles.f90:554-847)
 // ---------------------------------------------------------------------------
+// one stored point, read-only: a 32-byte load
+__device__ __forceinline__ Node64 ld_node(const Node64 *p) {
+    Node64 n;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(n.u), "=d"(n.v), "=d"(n.T), "=d"(n.q) : "l"(p));
+    return n;
+}
+
 // uf_interp_lin, particles.f90:767-847
 __device__ void interp_lin64(const DevBox &B, double x1, double x2, double x3, Interp &o, int &bad) {
     const DevGrid &g = B.g;
@@ -49,7 +56,6 @@ __device__ void interp_lin64(const DevBox &B, double x1, double x2, double x3, I
         wz[i] = (1.0 - fabs(x3 - zv) / g.dzu[kpt + 1]);
         wzw[i] = (1.0 - fabs(x3 - zwv) / g.dzw[kwpt + 1]);
     }
-    const double *fu = B.f[0], *fv = B.f[1], *fw = B.f[2], *fT = B.f[3], *fq = B.f[4];
     double u1 = 0.0, u2 = 0.0, u3 = 0.0, T = 0.0, q = 0.0;
     int ix = 0, iy = 0;
     for (int i = 0; i <= 1; ++i) {
@@ -57,21 +63,17 @@ __device__ void interp_lin64(const DevBox &B, double x1, double x2, double x3, I
             for (int k = 0; k <= 1; ++k) {
                 ix = ipt + i;
                 iy = jpt + j;
-                long long a = ext_index(g, kpt + k, iy, ix, bad);
+                const Node64 n = ld_node(B.f64 + ext_index(g, kpt + k, iy, ix, bad));
                 long long aw = ext_index(g, kwpt + k, iy, ix, bad);
-                u1 = u1 + __ldg(fu + a) * wx[i] * wy[j] * wz[k];
-                u2 = u2 + __ldg(fv + a) * wx[i] * wy[j] * wz[k];
-                u3 = u3 + __ldg(fw + aw) * wx[i] * wy[j] * wzw[k];
-                T = T + __ldg(fT + a) * wx[i] * wy[j] * wz[k];
-                q = q + __ldg(fq + a) * wx[i] * wy[j] * wz[k];
+                u1 = u1 + n.u * wx[i] * wy[j] * wz[k];
+                u2 = u2 + n.v * wx[i] * wy[j] * wz[k];
+                u3 = u3 + __ldg(B.fw64 + aw) * wx[i] * wy[j] * wzw[k];
+                T = T + n.T * wx[i] * wy[j] * wz[k];
+                q = q + n.q * wx[i] * wy[j] * wz[k];
             }
-            if (kpt == g.nnz) {
-                long long a = ext_index(g, kpt, iy, ix, bad);
-                u1 = __ldg(fu + a); u2 = __ldg(fv + a); T = __ldg(fT + a); q = __ldg(fq + a);
-            }
-            if (kpt == 0) {
-                long long a = ext_index(g, 1, iy, ix, bad);
-                u1 = __ldg(fu + a); u2 = __ldg(fv + a); T = __ldg(fT + a); q = __ldg(fq + a);
+            if (kpt == g.nnz || kpt == 0) {
+                const Node64 n = ld_node(B.f64 + ext_index(g, kpt == 0 ? 1 : kpt, iy, ix, bad));
+                u1 = n.u; u2 = n.v; T = n.T; q = n.q;
             }
         }
     }
@@ -95,20 +97,14 @@ __device__ __forceinline__ void lagrange6(double x, const double xn[6], int firs
     }
 }
 
-// uf_interp, particles.f90:554-765
-// one field value; TEXPATH: through the texture path (the same 8 bytes)
-template <bool TEXPATH>
-__device__ __forceinline__ double ld64(const double *f, unsigned long long tex, long long a) {
-    if (TEXPATH) {
-        const int2 v = tex1Dfetch<int2>((cudaTextureObject_t)tex, (int)a);
-        return __hiloint2double(v.y, v.x);
-    }
-    return __ldg(f + a);
-}
-
-// TEX: the first three x columns of the stencil through the texture path (its
-// own L1 data pipe)
-template <bool TEX>
+// uf_interp, particles.f90:554-765.
+//
+// Bound by instruction issue and the FP64 pipe: 216 points of 3 multiplies and
+// an add for each of 5 fields, 4320 operations that the order of the reference
+// does not let share anything.  What is left to save is around them: a point
+// is one 32-byte load and one of w, at 32-bit offsets, and the j and i loops
+// are unrolled so that no weight moves between registers (k stays rolled).
+// FIGURES
 __device__ void interp6_64(const DevBox &B, double x1, double x2, double x3, Interp &o, int &bad) {
     const DevGrid &g = B.g;
     const int nnz = g.nnz;
@@ -163,10 +159,10 @@ __device__ void interp6_64(const DevBox &B, double x1, double x2, double x3, Int
         }
         lagrange6(x3, zn, first, last, wzw);
     }
-    // index offsets per axis (x: periodic image of column nnx+4 and clamping
-    // of anything outside the padded array, as ext_index does per read)
-    long long xo[6];
-    int yo[6];
+    // point offsets per axis (x: periodic image of column nnx+4 and clamping
+    // of anything outside the padded array, as ext_index does per read); the
+    // padded array has at most 2^31 - 1 points
+    unsigned xo[6], yo[6];
 #pragma unroll
     for (int a = 0; a < 6; ++a) {
         int ix = ip3 + (a - 2), iy = jp3 + (a - 2);
@@ -174,53 +170,35 @@ __device__ void interp6_64(const DevBox &B, double x1, double x2, double x3, Int
         if (g.periodic && iy > g.nny + 3) iy -= g.nny;
         if (ix < -1 || ix > g.nnx + 3) { bad = 1; ix = ix < -1 ? -1 : g.nnx + 3; }
         if (iy < -1 || iy > g.nny + 3) { bad = 1; iy = iy < -1 ? -1 : g.nny + 3; }
-        xo[a] = (long long)g.nz2 * g.ny5 * (ix + 1);
-        yo[a] = g.nz2 * (iy + 1);
+        xo[a] = (unsigned)(g.nz2 * g.ny5) * (unsigned)(ix + 1);
+        yo[a] = (unsigned)g.nz2 * (unsigned)(iy + 1);
         if (ku[a] < 0 || ku[a] > nnz + 1) { bad = 1; ku[a] = ku[a] < 0 ? 0 : nnz + 1; }
         if (kw[a] < 0 || kw[a] > nnz + 1) { bad = 1; kw[a] = kw[a] < 0 ? 0 : nnz + 1; }
     }
-    const double *fu = B.f[0], *fv = B.f[1], *fw = B.f[2], *fT = B.f[3], *fq = B.f[4];
+    const Node64 *f = B.f64;
+    const double *fw = B.fw64;
     double u1 = 0.0, u2 = 0.0, u3 = 0.0, T = 0.0, q = 0.0;
-    // reference order: k outer, j, i inner; k and j stay rolled, their
+    // reference order: k outer, j, i inner; k stays rolled, its
     // per-iteration values rotated through slot 0
 #pragma unroll 1
     for (int k = 0; k < 6; ++k) {
-        const int izuv = ku[0], izw = kw[0];
+        const unsigned izuv = (unsigned)ku[0], izw = (unsigned)kw[0];
         const double wk = wz[0], wkw = wzw[0];
-        double wyr[6];
-        int yor[6];
 #pragma unroll
-        for (int r = 0; r < 6; ++r) { wyr[r] = wy[r]; yor[r] = yo[r]; }
-#pragma unroll 1
         for (int j = 0; j < 6; ++j) {
-            const double wj = wyr[0];
-            const long long bu = izuv + yor[0], bw = izw + yor[0];
+            const double wj = wy[j];
+            const unsigned bu = izuv + yo[j], bw = izw + yo[j];
 #pragma unroll
             for (int i = 0; i < 6; ++i) {
                 const double wi = wx[i];
-                const long long a = bu + xo[i], aw = bw + xo[i];
-                double vu, vv, vw, vT, vq;
-                if (TEX && i < 3) {
-                    vu = ld64<true>(fu, B.tex_f64[0], a);
-                    vv = ld64<true>(fv, B.tex_f64[1], a);
-                    vw = ld64<true>(fw, B.tex_f64[2], aw);
-                    vT = ld64<true>(fT, B.tex_f64[3], a);
-                    vq = ld64<true>(fq, B.tex_f64[4], a);
-                } else {
-                    vu = ld64<false>(fu, 0, a);
-                    vv = ld64<false>(fv, 0, a);
-                    vw = ld64<false>(fw, 0, aw);
-                    vT = ld64<false>(fT, 0, a);
-                    vq = ld64<false>(fq, 0, a);
-                }
-                u1 = u1 + vu * wi * wj * wk;
-                u2 = u2 + vv * wi * wj * wk;
+                const Node64 n = ld_node(f + (bu + xo[i]));
+                const double vw = __ldg(fw + (bw + xo[i]));
+                u1 = u1 + n.u * wi * wj * wk;
+                u2 = u2 + n.v * wi * wj * wk;
                 u3 = u3 + vw * wi * wj * wkw;
-                T = T + vT * wi * wj * wk;
-                q = q + vq * wi * wj * wk;
+                T = T + n.T * wi * wj * wk;
+                q = q + n.q * wi * wj * wk;
             }
-#pragma unroll
-            for (int r = 0; r < 5; ++r) { wyr[r] = wyr[r + 1]; yor[r] = yor[r + 1]; }
         }
 #pragma unroll
         for (int r = 0; r < 5; ++r) {
@@ -235,8 +213,13 @@ __device__ void interp6_64(const DevBox &B, double x1, double x2, double x3, Int
 // launches: interpolation, droplet body with Gauss-Newton, deferred
 // Levenberg-Marquardt droplets.
 // ---------------------------------------------------------------------------
-template <int ILIN, int NT, bool TEX>
-__global__ void __launch_bounds__(NT)
+#ifndef IW
+#define IW 16
+#endif
+constexpr int kInterp64Warps = IW;   // resident warps per SM
+
+template <int ILIN, int NT>
+__global__ void __launch_bounds__(NT, ILIN == 1 ? 1 : kInterp64Warps * 32 / NT)
 k_interp64(DevBox *boxes, const Tile *tiles) {
     const Tile tl = tiles[blockIdx.x];
     const DevBox &B = boxes[tl.box];
@@ -248,7 +231,7 @@ k_interp64(DevBox *boxes, const Tile *tiles) {
     Interp I;
     int bad = 0;
     if (ILIN == 1) interp_lin64(B, S.x[0][s], S.x[1][s], S.x[2][s], I, bad);
-    else interp6_64<TEX>(B, S.x[0][s], S.x[1][s], S.x[2][s], I, bad);
+    else interp6_64(B, S.x[0][s], S.x[1][s], S.x[2][s], I, bad);
     O.uf[0][t] = I.uf[0];
     O.uf[1][t] = I.uf[1];
     O.uf[2][t] = I.uf[2];
@@ -287,9 +270,9 @@ k_be_defer64(DevBox *boxes, const __grid_constant__ DevParams P, StepIn in) {
 }
 
 // ---------------------------------------------------------------------------
-// RK3 stage (particles.f90:2845-2998), coefficients les.F:856-861
+// RK3 stage (particles.f90:2845-2998), coefficients les.F:856-861, after
+// k_interp64 (one kernel held 252 registers, 8 warps per SM)
 // ---------------------------------------------------------------------------
-template <int ILIN>
 __global__ void __launch_bounds__(kUpdateThreads)
 k_update_rk3_64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P, StepIn in) {
     const Tile tl = tiles[blockIdx.x];
@@ -329,9 +312,10 @@ k_update_rk3_64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevPar
         const long long multi = S.mult[s];
 
         Interp I;
-        int bad = 0;
-        if (ILIN == 1) interp_lin64(B, x[0], x[1], x[2], I, bad);
-        else interp6_64<false>(B, x[0], x[1], x[2], I, bad);
+        const int bad = B.key[t];
+        for (int a = 0; a < 3; ++a) I.uf[a] = O.uf[a][t];
+        I.Tf = O.Tf[t];
+        I.qinf = O.qinf[t];
         double Tf = I.Tf, qinf = I.qinf, rhoa;
         if (p.iexner == 1) {
             Tf = Tf * exner64(p, p.surf_p, func_p_base64(p, p.surf_p, p.tsfcc1, x[2]));
@@ -382,13 +366,13 @@ k_update_rk3_64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevPar
         const int alive = apply_bcs(B, p, x, v, radius);
         if (bad) cnt.v[C_BAD]++;
         for (int a = 0; a < 3; ++a) {
-            O.x[a][t] = x[a]; O.v[a][t] = v[a]; O.uf[a][t] = I.uf[a]; O.vold[a][t] = vold[a];
+            O.x[a][t] = x[a]; O.v[a][t] = v[a]; O.vold[a][t] = vold[a];
             O.xrhs[a][t] = xrhs[a]; O.vrhs[a][t] = vrhs[a];
         }
         O.Tp[t] = Tp; O.r[t] = radius; O.m_s[t] = m_s; O.kap[t] = kap; O.rc[t] = S.rc[s];
         O.res[t] = res; O.actres[t] = S.actres[s]; O.numact[t] = S.numact[s]; O.mult[t] = multi;
         O.lid[t] = S.lid[s];
-        O.Tf[t] = Tf; O.qinf[t] = qinf; O.qstar[t] = qstar; O.Tpold[t] = Tpold; O.rold[t] = rold;
+        O.Tf[t] = Tf; O.qstar[t] = qstar; O.Tpold[t] = Tpold; O.rold[t] = rold;
         O.Tprhs_s[t] = Tprhs_s; O.Tprhs_L[t] = Tprhs_L; O.radrhs[t] = radrhs;
         int key;
         if (alive >= 10) {
@@ -431,17 +415,15 @@ __global__ void k_payload64(DevBox *boxes, const Tile *tiles, const __grid_const
 // launchers
 // ---------------------------------------------------------------------------
 void launch_update_be64(int ilin, int nt, DevBox *boxes, const Tile *tiles, int ntiles, int nbox,
-                        const DevParams &P, StepIn in, cudaStream_t st, bool tex) {
+                        const DevParams &P, StepIn in, cudaStream_t st) {
     if (ntiles <= 0) return;
     if (nt == 256) {
-        if (ilin == 1) k_interp64<1, 256, false><<<ntiles, 256, 0, st>>>(boxes, tiles);
-        else if (tex) k_interp64<0, 256, true><<<ntiles, 256, 0, st>>>(boxes, tiles);
-        else k_interp64<0, 256, false><<<ntiles, 256, 0, st>>>(boxes, tiles);
+        if (ilin == 1) k_interp64<1, 256><<<ntiles, 256, 0, st>>>(boxes, tiles);
+        else k_interp64<0, 256><<<ntiles, 256, 0, st>>>(boxes, tiles);
         k_be64<256><<<ntiles, 256, 0, st>>>(boxes, tiles, P, in);
     } else {
-        if (ilin == 1) k_interp64<1, 128, false><<<ntiles, 128, 0, st>>>(boxes, tiles);
-        else if (tex) k_interp64<0, 128, true><<<ntiles, 128, 0, st>>>(boxes, tiles);
-        else k_interp64<0, 128, false><<<ntiles, 128, 0, st>>>(boxes, tiles);
+        if (ilin == 1) k_interp64<1, 128><<<ntiles, 128, 0, st>>>(boxes, tiles);
+        else k_interp64<0, 128><<<ntiles, 128, 0, st>>>(boxes, tiles);
         k_be64<128><<<ntiles, 128, 0, st>>>(boxes, tiles, P, in);
     }
     k_be_defer64<<<dim3(kDeferBlocks, nbox), kUpdateThreads, 0, st>>>(boxes, P, in);
@@ -450,10 +432,10 @@ void launch_update_be64(int ilin, int nt, DevBox *boxes, const Tile *tiles, int 
 void launch_update_rk3_64(int ilin, DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P,
                           StepIn in, cudaStream_t st) {
     if (ntiles <= 0) return;
-    if (ilin == 1)
-        k_update_rk3_64<1><<<ntiles, kUpdateThreads, 0, st>>>(boxes, tiles, P, in);
-    else
-        k_update_rk3_64<0><<<ntiles, kUpdateThreads, 0, st>>>(boxes, tiles, P, in);
+    static_assert(kUpdateThreads == 128, "one tile table for both kernels");
+    if (ilin == 1) k_interp64<1, 128><<<ntiles, 128, 0, st>>>(boxes, tiles);
+    else k_interp64<0, 128><<<ntiles, 128, 0, st>>>(boxes, tiles);
+    k_update_rk3_64<<<ntiles, kUpdateThreads, 0, st>>>(boxes, tiles, P, in);
 }
 
 void launch_payload64(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P, double dt,

@@ -37,7 +37,7 @@ struct StepIn {
 
 // FP64, reference operation order (ntlp_fp64.cu)
 void launch_update_be64(int ilin, int nt, DevBox *boxes, const Tile *tiles, int ntiles, int nbox,
-                        const DevParams &P, StepIn in, cudaStream_t st, bool tex);
+                        const DevParams &P, StepIn in, cudaStream_t st);
 void launch_update_rk3_64(int ilin, DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P,
                           StepIn in, cudaStream_t st);
 void launch_payload64(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P, double dt,
@@ -111,9 +111,13 @@ void launch_finish(DevBox *boxes, int nbox, cudaStream_t st);
 void launch_reset_step(DevBox *boxes, int nbox, cudaStream_t st);
 void launch_keys_initial(DevBox *boxes, const Tile *tiles, int ntiles, cudaStream_t st);
 
-// halo fill from the flow layout (fill_ext on one domain) and FP32 copies
-void launch_fill_ext(const double *flow, double *ext, const DevGrid &g, cudaStream_t st);
-void launch_pack_f32(const DevBox *host_box, float4 *f4, float *fw, cudaStream_t st);
+// the stored fields from arrays in device memory (u, v, w, T, q; a NULL array
+// leaves its field as it is): from the flow layout with the halo
+// (fill_ext on one domain), or from the halo-padded layout
+struct FieldSrc {
+    const double *p[5];
+};
+void launch_fill_fields(const DevBox &host_box, const FieldSrc &src, bool flow, cudaStream_t st);
 
 // download: position of each survivor in list order (scratch: (nlid + 1023) / 1024 ints)
 void launch_rank_alive(DevBox *boxes, int box, int *rank_by_lid, int nlid, int *scratch, cudaStream_t st);

@@ -137,12 +137,11 @@ __device__ void interp6_mixed(const DevBox &B, double x1, double x2, double x3, 
 #pragma unroll
         for (int r = 0; r < 5; ++r) wx[r] = wx[r + 1];
     }
-    const long long ridx = f32_ref_index(g);
-    o.uf[0] = B.f[0][ridx] + (double)su;
-    o.uf[1] = B.f[1][ridx] + (double)sv;
-    o.uf[2] = B.f[2][ridx] + (double)sw;
-    o.Tf = B.f[3][ridx] + (double)sT;
-    o.qinf = B.f[4][ridx] + (double)sq;
+    o.uf[0] = B.ref[0] + (double)su;
+    o.uf[1] = B.ref[1] + (double)sv;
+    o.uf[2] = B.ref[2] + (double)sw;
+    o.Tf = B.ref[3] + (double)sT;
+    o.qinf = B.ref[4] + (double)sq;
 }
 
 __device__ void interp_lin_mixed(const DevBox &B, double x1, double x2, double x3, Interp &o, int &bad) {
@@ -195,12 +194,11 @@ __device__ void interp_lin_mixed(const DevBox &B, double x1, double x2, double x
             }
         }
     }
-    const long long ridx = f32_ref_index(g);
-    o.uf[0] = B.f[0][ridx] + (double)u1;
-    o.uf[1] = B.f[1][ridx] + (double)u2;
-    o.uf[2] = B.f[2][ridx] + (double)u3;
-    o.Tf = B.f[3][ridx] + (double)T;
-    o.qinf = B.f[4][ridx] + (double)q;
+    o.uf[0] = B.ref[0] + (double)u1;
+    o.uf[1] = B.ref[1] + (double)u2;
+    o.uf[2] = B.ref[2] + (double)u3;
+    o.Tf = B.ref[3] + (double)T;
+    o.qinf = B.ref[4] + (double)q;
 }
 
 template <int ILIN, int NT, bool TEX>
@@ -503,9 +501,8 @@ __global__ void __launch_bounds__(kBlockThreads, 4) k_interp_block(DevBox *boxes
     __shared__ StageCtx sc;
     if (threadIdx.x == 0) {
         const DevState &O = B.st[1 - B.cur];
-        const long long ridx = f32_ref_index(g);
         sc.dx = g.dx; sc.dy = g.dy; sc.lut_scale = g.lut_scale;
-        for (int q = 0; q < 5; ++q) sc.ref[q] = B.f[q][ridx];
+        for (int q = 0; q < 5; ++q) sc.ref[q] = B.ref[q];
         sc.zz = g.zz; sc.z = g.z; sc.lut_zz = g.lut_zz; sc.lut_z = g.lut_z;
         for (int a = 0; a < 3; ++a) sc.xp[a] = S.x[a];
         sc.perm = B.perm;

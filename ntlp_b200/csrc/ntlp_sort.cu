@@ -10,6 +10,8 @@
 // the scatter uses atomics.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "ntlp_dev.cuh"
 #include "ntlp_kernels.h"
 
@@ -285,65 +287,144 @@ void launch_keys_initial(DevBox *boxes, const Tile *tiles, int ntiles, cudaStrea
     if (ntiles > 0) k_keys_initial<<<ntiles, kUpdateThreads, 0, st>>>(boxes, tiles);
 }
 
-// ---- halo fill: flow layout u(1:nnx,1:nny,0:nnz+1) -> ext(0:nnz+1,-1:nny+3,-1:nnx+3)
-// 32x32 tiles of the (i, k) plane per output row j, staged through shared
-// memory so both the x-fastest read and the z-fastest write are coalesced.
-__global__ void k_fill_ext(const double *__restrict__ flow, double *__restrict__ ext, DevGrid g) {
-    __shared__ double tile[32][33];
+// ---- stored fields -----------------------------------------------------------
+// one field value (q: u, v, w, T, q) or all of a point, in the path's form
+struct StoreF64 {
+    Node64 *f;
+    double *w;
+    __device__ __forceinline__ void one(int q, long long o, double v) const {
+        if (q == 2) w[o] = v;
+        else (&f[o].u)[q < 2 ? q : q - 1] = v;
+    }
+    __device__ __forceinline__ void all(long long o, const double v[5]) const {
+        asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(f + o), "d"(v[0]), "d"(v[1]), "d"(v[3]),
+                     "d"(v[4])
+                     : "memory");
+        w[o] = v[2];
+    }
+};
+struct StoreF32 {   // deviations from the reference values
+    float4 *f;
+    float *w;
+    double ref[5];
+    __device__ __forceinline__ void one(int q, long long o, double v) const {
+        const float d = (float)(v - ref[q]);
+        if (q == 2) w[o] = d;
+        else (&f[o].x)[q < 2 ? q : q - 1] = d;
+    }
+    __device__ __forceinline__ void all(long long o, const double v[5]) const {
+        f[o] = make_float4((float)(v[0] - ref[0]), (float)(v[1] - ref[1]), (float)(v[3] - ref[3]),
+                           (float)(v[4] - ref[4]));
+        w[o] = (float)(v[2] - ref[2]);
+    }
+};
+
+// the mixed path's store: reference values read from the source arrays
+// (element ridx of each), and kept in B.ref by the grid's first thread
+__device__ __forceinline__ StoreF32 store32(const DevBox &B, const FieldSrc &s, long long ridx, bool first) {
+    StoreF32 S;
+    S.f = const_cast<float4 *>(B.f4);
+    S.w = const_cast<float *>(B.fw);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+        S.ref[q] = s.p[q] ? s.p[q][ridx] : 0.0;
+        if (first && s.p[q]) const_cast<double *>(B.ref)[q] = S.ref[q];
+    }
+    return S;
+}
+
+// flow layout u(1:nnx,1:nny,0:nnz+1) -> stored points (0:nnz+1,-1:nny+3,-1:nnx+3).
+// A block takes the fields of a 32x32 tile of the (i, k) plane of one output
+// row j through shared memory, so both the x-fastest reads and the z-fastest
+// writes are coalesced.  HBM-bound: every value is read once (plus halos)
+// and every point written once.  A step of 256^3 fields in device memory (copy,
+// five halo fills and the FP32 pack before): FIGURES
+template <class Store>
+__device__ __forceinline__ void fill_tile(const FieldSrc &s, const DevGrid &g, const Store &S, double (*tile)[32][33]) {
     const int j = (int)blockIdx.z - 1;                 // -1 .. nny+3
-    const int i0 = (int)blockIdx.x * 32 - 1;           // ext i of tile start
+    const int i0 = (int)blockIdx.x * 32 - 1;           // i of the tile's start
     const int k0 = (int)blockIdx.y * 32;
     const int jsrc = ((j - 1) % g.nny + g.nny) % g.nny;  // 0-based source row
-    // load: threads along i (x fastest in flow)
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        int k = k0 + r;
-        int i = i0 + (int)threadIdx.x;
-        if (k <= g.nnz + 1 && i <= g.nnx + 3) {
-            int isrc = ((i - 1) % g.nnx + g.nnx) % g.nnx;
-            tile[r][threadIdx.x] = flow[(long long)isrc + (long long)g.nnx * ((long long)jsrc + (long long)g.nny * k)];
+    const int i = i0 + (int)threadIdx.x;
+    const int isrc = ((i - 1) % g.nnx + g.nnx) % g.nnx;
+    bool every = true;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+        const double *p = s.p[q];
+        every = every && p != nullptr;
+        if (p == nullptr) continue;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int k = k0 + (int)threadIdx.y + 8 * r;
+            if (k <= g.nnz + 1 && i <= g.nnx + 3)
+                tile[q][threadIdx.y + 8 * r][threadIdx.x] =
+                    __ldcs(p + isrc + (long long)g.nnx * (jsrc + (long long)g.nny * k));
         }
     }
     __syncthreads();
-    // store: threads along k (z fastest in ext)
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        int i = i0 + r;
-        int k = k0 + (int)threadIdx.x;
-        if (k <= g.nnz + 1 && i <= g.nnx + 3) {
-            long long o = (long long)k + (long long)g.nz2 * ((long long)(j + 1) + (long long)g.ny5 * (i + 1));
-            ext[o] = tile[threadIdx.x][r];
+    const int k = k0 + (int)threadIdx.x;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int io = i0 + (int)threadIdx.y + 8 * r;
+        if (k > g.nnz + 1 || io > g.nnx + 3) continue;
+        const long long o = (long long)k + (long long)g.nz2 * ((long long)(j + 1) + (long long)g.ny5 * (io + 1));
+        if (every) {
+            double v[5];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) v[q] = tile[q][threadIdx.x][threadIdx.y + 8 * r];
+            S.all(o, v);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 5; ++q)
+                if (s.p[q]) S.one(q, o, tile[q][threadIdx.x][threadIdx.y + 8 * r]);
         }
     }
 }
 
-void launch_fill_ext(const double *flow, double *ext, const DevGrid &g, cudaStream_t st) {
-    dim3 grid((g.nnx + 5 + 31) / 32, (g.nnz + 2 + 31) / 32, g.nny + 5);
-    dim3 block(32, 8);
-    k_fill_ext<<<grid, block, 0, st>>>(flow, ext, g);
-}
-
-// FP32 copies for the mixed path: (u, v, T, q) packed per point as float4,
-// w separately, each as the deviation from its value at point (1,1,1).
-__global__ void k_pack_f32(const double *__restrict__ u, const double *__restrict__ v,
-                           const double *__restrict__ w, const double *__restrict__ T,
-                           const double *__restrict__ q, float4 *__restrict__ f4, float *__restrict__ fw,
-                           long long n, long long ridx) {
-    const double ru = u[ridx], rv = v[ridx], rw = w[ridx], rT = T[ridx], rq = q[ridx];
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (; i < n; i += stride) {
-        f4[i] = make_float4((float)(u[i] - ru), (float)(v[i] - rv), (float)(T[i] - rT), (float)(q[i] - rq));
-        fw[i] = (float)(w[i] - rw);
+template <bool MIXED>
+__global__ void __launch_bounds__(256) k_fill_flow(const __grid_constant__ DevBox B, FieldSrc s) {
+    __shared__ double tile[5][32][33];
+    if constexpr (MIXED) {
+        const bool first = blockIdx.x + blockIdx.y + blockIdx.z == 0 && threadIdx.x + threadIdx.y == 0;
+        fill_tile(s, B.g, store32(B, s, (long long)B.g.nnx * B.g.nny, first), tile);   // (i, j, k) = (1, 1, 1)
+    } else {
+        fill_tile(s, B.g, StoreF64{const_cast<Node64 *>(B.f64), const_cast<double *>(B.fw64)}, tile);
     }
 }
 
-void launch_pack_f32(const DevBox *hb, float4 *f4, float *fw, cudaStream_t st) {
-    const DevGrid &g = hb->g;
+// halo-padded layout, the stored order already
+template <bool MIXED>
+__global__ void __launch_bounds__(256) k_fill_ext(const __grid_constant__ DevBox B, FieldSrc s, long long n) {
+    const bool every = s.p[0] && s.p[1] && s.p[2] && s.p[3] && s.p[4];
+    auto put = [&](const auto &S) {
+        const long long stride = (long long)gridDim.x * blockDim.x;
+        for (long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x; o < n; o += stride) {
+            if (every) {
+                const double v[5] = {s.p[0][o], s.p[1][o], s.p[2][o], s.p[3][o], s.p[4][o]};
+                S.all(o, v);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 5; ++q)
+                    if (s.p[q]) S.one(q, o, s.p[q][o]);
+            }
+        }
+    };
+    if constexpr (MIXED) put(store32(B, s, f32_ref_index(B.g), blockIdx.x + threadIdx.x == 0));
+    else put(StoreF64{const_cast<Node64 *>(B.f64), const_cast<double *>(B.fw64)});
+}
+
+void launch_fill_fields(const DevBox &B, const FieldSrc &s, bool flow, cudaStream_t st) {
+    const DevGrid &g = B.g;
+    if (flow) {
+        const dim3 grid((g.nnx + 5 + 31) / 32, (g.nnz + 2 + 31) / 32, g.nny + 5), block(32, 8);
+        if (B.f4) k_fill_flow<true><<<grid, block, 0, st>>>(B, s);
+        else k_fill_flow<false><<<grid, block, 0, st>>>(B, s);
+        return;
+    }
     const long long n = (long long)g.nz2 * g.ny5 * g.nx5;
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    if (blocks > 0)
-        k_pack_f32<<<blocks, 256, 0, st>>>(hb->f[0], hb->f[1], hb->f[2], hb->f[3], hb->f[4], f4, fw, n,
-                                            f32_ref_index(g));
+    const int blocks = (int)std::min<long long>((n + 255) / 256, 148 * 16);
+    if (B.f4) k_fill_ext<true><<<blocks, 256, 0, st>>>(B, s, n);
+    else k_fill_ext<false><<<blocks, 256, 0, st>>>(B, s, n);
 }
 
 // ---- download: list-order position of every survivor -----------------------
