@@ -8,7 +8,7 @@
 //              tallies, boundaries, new cell key, deposition payload);
 //              deferred Levenberg-Marquardt droplets
 //   sort       histogram + scan + scatter + per-cell lid order
-//   finish     adopt the new buffer and order, count survivors
+//   finish     adopt the new buffer, count survivors
 // particle_coupling_update adds the deposition.  Because every per-step
 // decision (buffer parity, droplet counts) lives in device memory, the same
 // sequence can be recorded once as a CUDA graph and replayed.
@@ -101,7 +101,6 @@ struct ntlp_ctx {
     int n_dep_tiles[kDepVariants] = {};
     long long *tile_sums_d = nullptr;
     int *box_first_tile_d = nullptr;
-    int *any_big_d = nullptr;
     int *overflow_list_d = nullptr;   // mixed deposition: tiles left to the global-memory kernel
     void *small_arena = nullptr;
     SortPlan plan{};
@@ -341,7 +340,6 @@ void carve_box(Carver &cv, BoxHost &h, DevBox &B, bool mixed) {
     const size_t nsrc = (size_t)g.nz2 * g.sny * g.snx;   // nnodes, or with the +1 column/row of a subdomain
     for (int q = 0; q < 6; ++q) cv.take(&B.src[q], nsrc);
     cv.take(&B.err, 1);
-    cv.take(&B.big_cells, 1);
     cv.take(&B.defer, n);
     cv.take(&B.ndefer, 1);
     if (!g.periodic) {
@@ -849,7 +847,6 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
             for (int v = 0; v < kDepVariants; ++v) k.take(&c->dep_tiles_d[v], dpt[v].size());
             k.take(&c->tile_sums_d, ct.size());
             k.take(&c->box_first_tile_d, bft.size());
-            k.take(&c->any_big_d, 1);
             {
                 size_t mx = 0;
                 for (int v = 0; v < kDepVariants; ++v) mx = std::max(mx, dpt[v].size());
@@ -898,7 +895,6 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
     c->plan.tile_sums = c->tile_sums_d;
     c->plan.box_first_tile = c->box_first_tile_d;
     c->plan.nbox = nbox;
-    c->plan.any_big = c->any_big_d;
     if (cudaMallocHost((void **)&c->counters_h, sizeof(long long) * kNumCounters * nbox) != cudaSuccess ||
         cudaMallocHost((void **)&c->err_h, sizeof(int) * nbox) != cudaSuccess)
         return bail(fail(c, NTLP_ERR_NOMEM, "pinned counter buffer refused"));
@@ -1106,12 +1102,11 @@ int droplets_upload(ntlp_ctx *c, int b, const ntlp_droplets *d) {
     Tile *ctd = dtd + dtl.size();
     long long *sums = (long long *)(ctd + ctl.size());
     int *bft = (int *)(sums + ctl.size());
-    int *any_big = bft + 2;
     const int bf[2] = {0, (int)ctl.size()};
     CK(cudaMemcpyAsync(dtd, dtl.data(), dtl.size() * sizeof(Tile), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(ctd, ctl.data(), ctl.size() * sizeof(Tile), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(bft, bf, sizeof bf, cudaMemcpyHostToDevice, c->stream));
-    SortPlan plan{dtd, (int)dtl.size(), ctd, (int)ctl.size(), sums, bft, 1, any_big};
+    SortPlan plan{dtd, (int)dtl.size(), ctd, (int)ctl.size(), sums, bft, 1};
     launch_keys_initial(view, dtd, (int)dtl.size(), c->stream);
     launch_sort(view, plan, c->stream);
     launch_finish(view, 1, c->stream);
@@ -1136,7 +1131,7 @@ int droplets_download(ntlp_ctx *c, int b, ntlp_droplets *d) {
     const DevState &S = B.st[B.cur];
     // the list position of each droplet: its lid while every uploaded droplet
     // is alive, else its rank among the living; the slot table takes the
-    // array of the sort's result, which is dead between steps
+    // sort's scratch, which is free between steps
     int *slot = B.sorted;
     if (n != h.n_uploaded) launch_rank_alive(c->box_d, b, h.rank, h.n_uploaded, (int *)h.staging, c->stream);
     launch_slots(B.perm, S.lid, n != h.n_uploaded ? h.rank : nullptr, slot, n, c->stream);
@@ -1242,10 +1237,7 @@ int launch_step(ntlp_ctx *c, int kind, int istage, double dt, int32_t it, bool w
 // the host mirror follows the device's buffer flips
 void mirror_flip(ntlp_ctx *c, int nflips) {
     if (nflips & 1) {
-        for (auto &B : c->box) {
-            B.cur = 1 - B.cur;
-            std::swap(B.perm, B.sorted);
-        }
+        for (auto &B : c->box) B.cur = 1 - B.cur;
     }
 }
 

@@ -170,13 +170,13 @@ struct DevBox {
     int *key;              // [cap] new cell key of st[1-cur][t]
     int *cell_cnt;         // [ncells+2]
     int *cell_start;       // [ncells+3]
-    int *sorted;           // [cap] indices into st[1-cur], by cell then lid
+    int *sorted;           // [cap] sort scratch: indices into st[1-cur] by cell, unranked;
+                           // between steps free (slot table of a read-back)
     long long *counters;   // [kNumCounters]
     double *pflux;         // [nnz+1]
     long long *flux_fx;    // [2][nnz+1][kFluxLimbs]
     double *src[6];        // [nnodes] each, column layout
     int *err;              // device error word (0 = fine)
-    int *big_cells;        // this sort has cells of more than kSmallCell droplets
     double *img;           // periodic boxes: [6][img_count] image nodes (ix > nnx or iy > nny)
     double *cellsum;       // mixed boxes with many droplets per cell: [ncells][8 corners][6]
                            // per-cell source sums (nullptr: tiled deposition)

@@ -101,11 +101,8 @@ struct SortPlan {
     long long *tile_sums;    // [n_cell_tiles]
     const int *box_first_tile;  // [nbox+1] first cell tile of each box
     int nbox;
-    int *any_big;            // some box has cells above kSmallCell (set by k_cellsort)
 };
-constexpr int kSortLaunches = 7;   // kernels launched by launch_sort
-constexpr int kSmallCell = 32;     // cells up to this size are insertion-sorted by one thread
-constexpr int kRankBlocks = 1184;  // grid of the large-cell ranking (8 blocks per SM)
+constexpr int kSortLaunches = 5;   // kernels launched by launch_sort
 void launch_sort(DevBox *boxes, const SortPlan &plan, cudaStream_t st);
 void launch_finish(DevBox *boxes, int nbox, cudaStream_t st);
 void launch_reset_step(DevBox *boxes, int nbox, cudaStream_t st);

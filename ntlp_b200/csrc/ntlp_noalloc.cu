@@ -193,7 +193,6 @@ extern "C" int ntlp_coupling_noalloc(const ntlp_grid *grid, const ntlp_params *p
     B.cap = (int)n;
     B.n_alive = (int *)(S + kOffSmall);
     B.err = (int *)(S + kOffSmall) + 1;
-    B.big_cells = (int *)(S + kOffSmall) + 2;
     B.counters = (long long *)(S + kOffSmall + 64);
     B.pflux = (double *)(S + kOffFlux);
     B.flux_fx = (long long *)(S + kOffFlux + (kMaxNz + 1) * 8);
@@ -243,7 +242,6 @@ extern "C" int ntlp_coupling_noalloc(const ntlp_grid *grid, const ntlp_params *p
     plan.tile_sums = sums;
     plan.box_first_tile = box_first;
     plan.nbox = 1;
-    plan.any_big = (int *)(S + kOffSmall) + 3;
     launch_keys_initial(B_d, drop_tiles, nd, st);
     launch_sort(B_d, plan, st);
     launch_finish(B_d, 1, st);

@@ -3,7 +3,7 @@
 // After an update kernel has written every droplet's new cell key, the
 // droplets are bucketed by key (a counting sort: histogram, per-box
 // exclusive scan, scatter) and each cell's list is put in list order
-// (ascending lid).  The sorted index list becomes the next step's read
+// (ascending lid).  The ranked index list becomes the next step's read
 // permutation, and the cell offsets drive the deposition.  Keys are the
 // reference's binning (floor(x/dx)+1, minloc on zz), so cell membership is
 // exact; the per-cell lid order makes the layout deterministic even though
@@ -44,12 +44,8 @@ __global__ void k_scan_sums(DevBox *boxes, const Tile *tiles, long long *sums) {
 }
 
 // one block per box: exclusive scan of the box's tile sums, in place
-__global__ void k_scan_offsets(DevBox *boxes, const int *box_first_tile, long long *sums, int *any_big) {
+__global__ void k_scan_offsets(const int *box_first_tile, long long *sums) {
     const int b = blockIdx.x;
-    if (threadIdx.x == 0) {
-        *boxes[b].big_cells = 0;    // set again by k_cellsort
-        if (b == 0) *any_big = 0;
-    }
     const int a = box_first_tile[b], e = box_first_tile[b + 1];
     __shared__ long long carry;
     if (threadIdx.x == 0) carry = 0;
@@ -136,106 +132,68 @@ __global__ void k_scatter(DevBox *boxes, const Tile *tiles) {
     const int k = B.key[t];
     // counts down: the last droplet of a cell leaves its count at zero,
     // ready for the next step's histogram (the order inside a cell is
-    // k_cellsort's)
+    // k_cellrank's)
     const int pos = B.cell_start[k] + atomicSub(&B.cell_cnt[k], 1) - 1;
     B.sorted[pos] = t;
 }
 
 // ---- per-cell list order (ascending lid) -----------------------------------
-__global__ void k_cellsort(DevBox *boxes, const Tile *tiles, int *any_big) {
+// One thread per sorted position: its droplet's rank among its cell's lids
+// (ties, which unique lids never make, by position) is its place in the
+// cell.  The order goes into the previous permutation, which is dead
+// between the update and the finish, and becomes the new one.  The lids
+// of a block's own positions are in shared memory, so a cell's lanes read
+// them as broadcasts; only cells across its edges go to global memory.  O(n)
+// per droplet of a cell of n: bound by the gathers of key and lid at one
+// droplet per cell, by the loop at dozens.  It replaces an insertion sort in
+// global memory, one thread per cell: the whole sort of 2 M droplets at 31 per
+// cell took 0.71 ms, it takes 0.089 (16.8 M at one per cell: 0.44 -> 0.41).
+__global__ void __launch_bounds__(kUpdateThreads) k_cellrank(DevBox *boxes, const Tile *tiles) {
+    __shared__ int s_lid[kUpdateThreads];
     const Tile tl = tiles[blockIdx.x];
     const DevBox &B = boxes[tl.box];
-    const long long nb = nbuckets(B);
+    const int n = *B.n_alive;
+    if (tl.start >= n) return;
+    const int p = tl.start + threadIdx.x;
     const int *lid = B.st[1 - B.cur].lid;
-    for (int i = threadIdx.x; i < kScanTile; i += blockDim.x) {
-        const long long c = (long long)tl.start + i;
-        if (c >= nb) break;
-        if (c == nb - 1) continue;       // killed droplets: order irrelevant
-        const int a = B.cell_start[c], e = B.cell_start[c + 1];
-        if (e - a < 2) continue;
-        if (e - a > kSmallCell) {       // ranked by k_cellrank / k_cellcopy
-            *B.big_cells = 1;
-            *any_big = 1;
-            continue;
-        }
-        // insertion sort by lid (few droplets)
-        for (int p = a + 1; p < e; ++p) {
-            const int tv = B.sorted[p];
-            const int lv = lid[tv];
-            int q = p - 1;
-            while (q >= a && lid[B.sorted[q]] > lv) {
-                B.sorted[q + 1] = B.sorted[q];
-                --q;
-            }
-            B.sorted[q + 1] = tv;
-        }
-    }
-}
-
-// Cells with more than kSmallCell droplets (dense configurations: hundreds
-// per cell): one thread per sorted position counts the cell's droplets
-// with a smaller lid (ties, which unique lids never make, by position) and
-// writes its droplet to that rank in the previous permutation, which is
-// dead between the update and the finish; k_cellcopy then moves the ranked
-// ranges back.  O(n) per droplet instead of the O(n^2) insertion sort of
-// one thread per cell.
-// grid-stride over the droplet tiles: a fixed grid, so that a sort without
-// large cells costs two short launches
-__global__ void k_cellrank(DevBox *boxes, const Tile *tiles, int ntiles, const int *any_big) {
-    if (*any_big == 0) return;
-    for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
-        const Tile tl = tiles[ti];
-        const DevBox &B = boxes[tl.box];
-        if (*B.big_cells == 0) continue;
-        const int p = tl.start + threadIdx.x;
-        if (p >= *B.n_alive) continue;
-        const long long nb = nbuckets(B);
-        const int tv = B.sorted[p];
+    int tv = 0, lv = 0, a = 0, e = 0;
+    if (p < n) {
+        tv = B.sorted[p];
         const int c = B.key[tv];
-        if (c == nb - 1) continue;
-        const int a = B.cell_start[c], e = B.cell_start[c + 1];
-        if (e - a <= kSmallCell) continue;
-        const int *lid = B.st[1 - B.cur].lid;
-        const int lv = lid[tv];
-        int r = 0;
-        for (int q = a; q < e; ++q) {
+        lv = lid[tv];
+        a = B.cell_start[c];
+        e = B.cell_start[c + 1];
+        if (c == nbuckets(B) - 1) a = p, e = p + 1;   // killed droplets: any order
+    }
+    s_lid[threadIdx.x] = lv;
+    __syncthreads();
+    if (p >= n) return;
+    int r = 0;
+    if (e - a > 1) {
+        const int lo = max(a, tl.start), hi = min(e, tl.start + kUpdateThreads);
+        for (int q = a; q < lo; ++q) {
             const int lq = lid[B.sorted[q]];
+            r += lq <= lv;                             // before p
+        }
+        for (int q = lo; q < hi; ++q) {
+            const int lq = s_lid[q - tl.start];
             r += (lq < lv) || (lq == lv && q < p);
         }
-        B.perm[a + r] = tv;
+        for (int q = hi; q < e; ++q) r += lid[B.sorted[q]] < lv;
     }
-}
-
-__global__ void k_cellcopy(DevBox *boxes, const Tile *tiles, int ntiles, const int *any_big) {
-    if (*any_big == 0) return;
-    for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
-        const Tile tl = tiles[ti];
-        const DevBox &B = boxes[tl.box];
-        if (*B.big_cells == 0) continue;
-        const int p = tl.start + threadIdx.x;
-        if (p >= *B.n_alive) continue;
-        const long long nb = nbuckets(B);
-        const int c = B.key[B.sorted[p]];
-        if (c == nb - 1) continue;
-        if (B.cell_start[c + 1] - B.cell_start[c] <= kSmallCell) continue;
-        B.sorted[p] = B.perm[p];
-    }
+    B.perm[a + r] = tv;
 }
 
 void launch_sort(DevBox *boxes, const SortPlan &plan, cudaStream_t st) {
     k_scan_sums<<<plan.n_cell_tiles, 256, 0, st>>>(boxes, plan.cell_tiles, plan.tile_sums);
-    k_scan_offsets<<<plan.nbox, 1024, 0, st>>>(boxes, plan.box_first_tile, plan.tile_sums, plan.any_big);
+    k_scan_offsets<<<plan.nbox, 1024, 0, st>>>(plan.box_first_tile, plan.tile_sums);
     k_scan_local<<<plan.n_cell_tiles, kCellThreads, 0, st>>>(boxes, plan.cell_tiles, plan.tile_sums);
     k_scatter<<<plan.n_drop_tiles, kUpdateThreads, 0, st>>>(boxes, plan.drop_tiles);
-    k_cellsort<<<plan.n_cell_tiles, 256, 0, st>>>(boxes, plan.cell_tiles, plan.any_big);
-    const int g = plan.n_drop_tiles < kRankBlocks ? plan.n_drop_tiles : kRankBlocks;
-    if (g > 0) {
-        k_cellrank<<<g, kUpdateThreads, 0, st>>>(boxes, plan.drop_tiles, plan.n_drop_tiles, plan.any_big);
-        k_cellcopy<<<g, kUpdateThreads, 0, st>>>(boxes, plan.drop_tiles, plan.n_drop_tiles, plan.any_big);
-    }
+    if (plan.n_drop_tiles > 0)
+        k_cellrank<<<plan.n_drop_tiles, kUpdateThreads, 0, st>>>(boxes, plan.drop_tiles);
 }
 
-// ---- finish: flip buffers, adopt the sorted order, count survivors ---------
+// ---- finish: flip buffers, count survivors ---------------------------------
 __global__ void k_finish(DevBox *boxes, int nbox) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nbox) return;
@@ -245,9 +203,6 @@ __global__ void k_finish(DevBox *boxes, int nbox) {
     *B.n_alive = alive;
     B.counters[C_NUMPART] = alive;
     B.cur = 1 - B.cur;
-    int *tmp = B.perm;
-    B.perm = B.sorted;
-    B.sorted = tmp;
 }
 
 void launch_finish(DevBox *boxes, int nbox, cudaStream_t st) {
@@ -337,8 +292,8 @@ __device__ __forceinline__ StoreF32 store32(const DevBox &B, const FieldSrc &s, 
 // A block takes the fields of a 32x32 tile of the (i, k) plane of one output
 // row j through shared memory, so both the x-fastest reads and the z-fastest
 // writes are coalesced.  HBM-bound: every value is read once (plus halos)
-// and every point written once.  A step of 256^3 fields in device memory (copy,
-// five halo fills and the FP32 pack before): FIGURES
+// and every point written once.  The mixed fields of 256^3 in device memory
+// (copy, five halo fills and the FP32 pack before) took 1.1 ms, it takes 0.3.
 template <class Store>
 __device__ __forceinline__ void fill_tile(const FieldSrc &s, const DevGrid &g, const Store &S, double (*tile)[32][33]) {
     const int j = (int)blockIdx.z - 1;                 // -1 .. nny+3

@@ -40,3 +40,33 @@ def test_list_order_and_ranks(n, killed):
     for k, v in dev.items():
         assert np.array_equal(v.cpu().numpy(), host[k]), k
     s.close()
+
+
+# one cell of n droplets: ranking blocks hold 128 sorted positions
+@pytest.mark.parametrize("n", [1, 2, 127, 128, 129, 257, 1000])
+@pytest.mark.gpu
+@pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")
+def test_rank_within_a_cell(n):
+    import ntlp_b200
+    import pyoracle
+    case = small_case(n=n + 40, grid_n=(6, 5, 7), params=gen.default_params(icase=0))
+    d = clone(case.droplets)
+    g = case.grid
+    rng = np.random.Generator(np.random.Philox(5))
+    one = rng.permutation(n + 40)[:n]                      # the cell's droplets, spread over the list
+    for a, (lo, w) in enumerate(((2 * g["xl"] / 6, g["xl"] / 6), (2 * g["yl"] / 5, g["yl"] / 5),
+                                 (g["zz"][3], g["zz"][4] - g["zz"][3]))):
+        d["xp"][a][one] = lo + w * (0.3 + 0.4 * rng.random(n))
+    d["vp"][:, one] = 0.0
+    s = ntlp_b200.DropletStep(g, case.params, capacity=n + 40)
+    ext = case.ext()
+    s.set_fields_ext(ext)
+    s.set_droplets(d)
+    s.particle_update_BE(1e-4, 2)
+    o = pyoracle.Oracle(g, case.params, ext)
+    od = clone(d)
+    o.step_be(od, 1e-4, 2)
+    want, _ = o.coupling(od, 1e-4)                         # sums in list order: the ranks decide the bits
+    for q, got in enumerate(s.particle_coupling_update(1e-4)):
+        assert np.array_equal(np.asarray(got).view(np.int64), want[q].view(np.int64)), q
+    s.close()
