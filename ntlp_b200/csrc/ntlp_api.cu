@@ -1375,7 +1375,7 @@ int stats_run(ntlp_ctx *c, int b, bool radius_hist) {
         h.stats = w;
     }
     launch_stats(c->box_d, b, g, c->dp_d, h.stats, radius_hist, c->stream);
-    c->launches += 2;
+    c->launches += 3;
     CK(cudaGetLastError());
     return NTLP_OK;
 }

@@ -139,8 +139,9 @@ void launch_shift_existing(DevBox *boxes, int box, int n, int m, const int *rank
 void launch_halo_add(DevBox *boxes, int box, int axis, const double *in, long long n_per_q, cudaStream_t st);
 
 // particle_xy_stats and radius_histogram of one box (ntlp_stats.cu)
-constexpr int kStatCols = 128;      // columns per tile (one block)
+constexpr int kStatCols = 64;       // columns per tile (one block)
 constexpr int kStatThreads = 256;
+constexpr int kStatWarps = kStatThreads / 32;
 constexpr int kS0N = 20;            // 0th-order values per partial
 struct StatsScratch {
     double *colsum;                 // [(nnx+1)(nny+1)] LWP per column
