@@ -886,6 +886,8 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
     if (!bt.empty())
         bad |= cudaMemcpyAsync(c->blk_tiles_d, bt.data(), bt.size() * sizeof(Tile), cudaMemcpyHostToDevice,
                                c->stream) != cudaSuccess;
+    // empty between depositions: k_fold clears it
+    bad |= cudaMemsetAsync(c->overflow_list_d, 0, sizeof(int), c->stream) != cudaSuccess;
     bad |= cudaMemcpyAsync(c->dp_d, &c->dp, sizeof(DevParams), cudaMemcpyHostToDevice, c->stream) != cudaSuccess;
     if (bad) return bail(fail(c, NTLP_ERR_CUDA, "uploading the tile tables failed"));
     c->plan.drop_tiles = c->drop_tiles_d[0];

@@ -300,6 +300,7 @@ __device__ __noinline__ void node_global64(const DevBox &B, const DevParams &p, 
 // Dense boxes (mixed): every cell's 8 corner sums S_o once, one thread per
 // (cell, corner) -- grid.y = box, grid-stride over cells x 8
 __global__ void k_cellsums32(DevBox *boxes, const __grid_constant__ DevParams P) {
+    step_kernel_begin();
     const DevBox &B = boxes[blockIdx.y];
     if (B.cellsum == nullptr) return;
     const long long total = B.g.ncells * 8;
@@ -316,6 +317,7 @@ __global__ void k_cellsums32(DevBox *boxes, const __grid_constant__ DevParams P)
 
 // Dense boxes (mixed): every output node from the cell sums
 __global__ void k_nodes_dense32(DevBox *boxes) {
+    step_kernel_begin();
     const DevBox &B = boxes[blockIdx.y];
     if (B.cellsum == nullptr) return;
     const DevGrid &g = B.g;
@@ -348,7 +350,10 @@ __device__ __forceinline__ void store_node(const DevBox &B, int ix, int iy, int 
 // Periodic boxes: the fold of particle_coupling_exchange on the nodes
 // with ix <= 2 or iy <= 2, from their own image (in the sources) and the
 // image nodes, in node_fold's order; grid.y = box
-__global__ void k_fold(DevBox *boxes) {
+__global__ void k_fold(DevBox *boxes, int *overflow_list) {
+    step_kernel_begin();
+    // the tiles listed for k_deposit_overflow32 are done: an empty list for the next deposition
+    if (overflow_list != nullptr && blockIdx.x + blockIdx.y + threadIdx.x == 0) overflow_list[0] = 0;
     const DevBox &B = boxes[blockIdx.y];
     const DevGrid &g = B.g;
     if (!g.periodic || B.img == nullptr || B.cellsum != nullptr) return;
@@ -441,6 +446,7 @@ __device__ __forceinline__ int tile_columns(const DevBox &B, int x0, int y0, int
 template <int TX, int TY, int TZ>
 __global__ void __launch_bounds__(kDepositThreads, 2)
 k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P) {
+    step_kernel_begin();
     static_assert(TX * TY * TZ == kDepositThreads, "one thread per node of the tile");
     constexpr int COLS = (TX + 1) * (TY + 1), CSW = TZ + 2, CAP = kDepCap64;
     extern __shared__ __align__(16) unsigned char sm[];
@@ -543,6 +549,7 @@ template <int kDepTX, int kDepTY, int kDepTZ>
 __global__ void __launch_bounds__(kDepositThreads, 4)
 k_deposit_tiled(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P, int *overflow_list,
                 int any_dense) {
+    step_kernel_begin<false>();
     static_assert(kDepTX * kDepTY * kDepTZ == kDepositThreads, "one thread per node of the tile");
     constexpr int kDepCols = (kDepTX + 1) * (kDepTY + 1);
     constexpr int kDepCSW = kDepTZ + 2;
@@ -646,6 +653,7 @@ k_deposit_tiled(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevPar
 template <int kDepTX, int kDepTY, int kDepTZ>
 __global__ void __launch_bounds__(kDepositThreads)
 k_deposit_overflow32(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P, const int *overflow_list) {
+    step_kernel_begin();
     const int n = overflow_list[0];
     for (int e = blockIdx.x; e < n; e += gridDim.x) {
         const Tile tl = tiles[overflow_list[1 + e]];

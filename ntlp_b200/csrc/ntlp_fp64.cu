@@ -221,6 +221,7 @@ constexpr int kInterp64Warps = 16;   // resident warps per SM
 template <int ILIN, int NT>
 __global__ void __launch_bounds__(NT, ILIN == 1 ? 1 : kInterp64Warps * 32 / NT)
 k_interp64(DevBox *boxes, const Tile *tiles) {
+    step_kernel_begin();
     const Tile tl = tiles[blockIdx.x];
     const DevBox &B = boxes[tl.box];
     const int t = tl.start + threadIdx.x;
@@ -245,6 +246,7 @@ k_interp64(DevBox *boxes, const Tile *tiles) {
 template <int NT>
 __global__ void __launch_bounds__(NT, 768 / NT)
 k_be64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P, StepIn in) {
+    step_kernel_begin();
     const Tile tl = tiles[blockIdx.x];
     const DevBox &B = boxes[tl.box];
     Counts cnt;
@@ -258,6 +260,7 @@ k_be64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P, St
 // Levenberg-Marquardt fallback (grid.y = box)
 __global__ void __launch_bounds__(kUpdateThreads)
 k_be_defer64(DevBox *boxes, const __grid_constant__ DevParams P, StepIn in) {
+    step_kernel_begin();
     const DevBox &B = boxes[blockIdx.y];
     Counts cnt;
     for (int k = 0; k < kNumCounters; ++k) cnt.v[k] = 0;
@@ -275,6 +278,7 @@ k_be_defer64(DevBox *boxes, const __grid_constant__ DevParams P, StepIn in) {
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kUpdateThreads)
 k_update_rk3_64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P, StepIn in) {
+    step_kernel_begin();
     const Tile tl = tiles[blockIdx.x];
     const DevBox &B = boxes[tl.box];
     const DevParams &p = P;
@@ -418,24 +422,24 @@ void launch_update_be64(int ilin, int nt, DevBox *boxes, const Tile *tiles, int 
                         const DevParams &P, StepIn in, cudaStream_t st) {
     if (ntiles <= 0) return;
     if (nt == 256) {
-        if (ilin == 1) k_interp64<1, 256><<<ntiles, 256, 0, st>>>(boxes, tiles);
-        else k_interp64<0, 256><<<ntiles, 256, 0, st>>>(boxes, tiles);
-        k_be64<256><<<ntiles, 256, 0, st>>>(boxes, tiles, P, in);
+        if (ilin == 1) launch_step_kernel(k_interp64<1, 256>, ntiles, 256, 0, st, boxes, tiles);
+        else launch_step_kernel(k_interp64<0, 256>, ntiles, 256, 0, st, boxes, tiles);
+        launch_step_kernel(k_be64<256>, ntiles, 256, 0, st, boxes, tiles, P, in);
     } else {
-        if (ilin == 1) k_interp64<1, 128><<<ntiles, 128, 0, st>>>(boxes, tiles);
-        else k_interp64<0, 128><<<ntiles, 128, 0, st>>>(boxes, tiles);
-        k_be64<128><<<ntiles, 128, 0, st>>>(boxes, tiles, P, in);
+        if (ilin == 1) launch_step_kernel(k_interp64<1, 128>, ntiles, 128, 0, st, boxes, tiles);
+        else launch_step_kernel(k_interp64<0, 128>, ntiles, 128, 0, st, boxes, tiles);
+        launch_step_kernel(k_be64<128>, ntiles, 128, 0, st, boxes, tiles, P, in);
     }
-    k_be_defer64<<<dim3(kDeferBlocks, nbox), kUpdateThreads, 0, st>>>(boxes, P, in);
+    launch_step_kernel(k_be_defer64, dim3(kDeferBlocks, nbox), kUpdateThreads, 0, st, boxes, P, in);
 }
 
 void launch_update_rk3_64(int ilin, DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P,
                           StepIn in, cudaStream_t st) {
     if (ntiles <= 0) return;
     static_assert(kUpdateThreads == 128, "one tile table for both kernels");
-    if (ilin == 1) k_interp64<1, 128><<<ntiles, 128, 0, st>>>(boxes, tiles);
-    else k_interp64<0, 128><<<ntiles, 128, 0, st>>>(boxes, tiles);
-    k_update_rk3_64<<<ntiles, kUpdateThreads, 0, st>>>(boxes, tiles, P, in);
+    if (ilin == 1) launch_step_kernel(k_interp64<1, 128>, ntiles, 128, 0, st, boxes, tiles);
+    else launch_step_kernel(k_interp64<0, 128>, ntiles, 128, 0, st, boxes, tiles);
+    launch_step_kernel(k_update_rk3_64, ntiles, kUpdateThreads, 0, st, boxes, tiles, P, in);
 }
 
 void launch_payload64(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P, double dt,
@@ -447,8 +451,7 @@ void launch_payload64(DevBox *boxes, const Tile *tiles, int ntiles, const DevPar
 template <int V>
 static void dep64(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P, cudaStream_t st) {
     constexpr int TX = kDepShape[V][0], TY = kDepShape[V][1], TZ = kDepShape[V][2];
-    k_deposit64<TX, TY, TZ>
-        <<<ntiles, kDepositThreads, dep_smem_bytes(false, TX, TY, TZ), st>>>(boxes, tiles, P);
+    launch_step_kernel(k_deposit64<TX, TY, TZ>, ntiles, kDepositThreads, dep_smem_bytes(false, TX, TY, TZ), st, boxes, tiles, P);
 }
 
 template <int V>
@@ -472,7 +475,7 @@ void launch_deposit64(int variant, DevBox *boxes, const Tile *tiles, int ntiles,
     if (variant == 1) dep64<1>(boxes, tiles, ntiles, P, st);
     else if (variant == 2) dep64<2>(boxes, tiles, ntiles, P, st);
     else dep64<0>(boxes, tiles, ntiles, P, st);
-    if (nbox > 0) k_fold<<<dim3(kFoldBlocks, nbox), 256, 0, st>>>(boxes);
+    if (nbox > 0) launch_step_kernel(k_fold, dim3(kFoldBlocks, nbox), 256, 0, st, boxes, nullptr);
 }
 
 }  // namespace ntlp

@@ -204,6 +204,7 @@ __device__ void interp_lin_mixed(const DevBox &B, double x1, double x2, double x
 template <int ILIN, int NT, bool TEX>
 __global__ void __launch_bounds__(NT, 512 / NT)
 k_interp_mixed(DevBox *boxes, const Tile *tiles) {
+    step_kernel_begin();
     const Tile tl = tiles[blockIdx.x];
     const DevBox &B = boxes[tl.box];
     const int t = tl.start + threadIdx.x;
@@ -397,6 +398,7 @@ __device__ __forceinline__ bool interp6_staged(const StageCtx &C, const float4 *
 
 template <int KB>
 __global__ void __launch_bounds__(kBlockThreads, 4) k_interp_block(DevBox *boxes, const Tile *tiles) {
+    step_kernel_begin<false>();
     using D = StageDims<KB>;
     constexpr int ZS = D::ZS, ZSW = D::ZSW, NLEV = D::NLEV;
     constexpr int NT = kBlockThreads;
@@ -567,10 +569,10 @@ void prepare_interp_block() {
 
 static void launch_interp_block(int kb, DevBox *boxes, const Tile *tiles, int ntiles, cudaStream_t st) {
     const int sm = interp_block_smem(kb);
-    if (kb == 4) k_interp_block<4><<<ntiles, kBlockThreads, sm, st>>>(boxes, tiles);
-    else if (kb == 16) k_interp_block<16><<<ntiles, kBlockThreads, sm, st>>>(boxes, tiles);
-    else if (kb == 32) k_interp_block<32><<<ntiles, kBlockThreads, sm, st>>>(boxes, tiles);
-    else k_interp_block<8><<<ntiles, kBlockThreads, sm, st>>>(boxes, tiles);
+    if (kb == 4) launch_step_kernel(k_interp_block<4>, ntiles, kBlockThreads, sm, st, boxes, tiles);
+    else if (kb == 16) launch_step_kernel(k_interp_block<16>, ntiles, kBlockThreads, sm, st, boxes, tiles);
+    else if (kb == 32) launch_step_kernel(k_interp_block<32>, ntiles, kBlockThreads, sm, st, boxes, tiles);
+    else launch_step_kernel(k_interp_block<8>, ntiles, kBlockThreads, sm, st, boxes, tiles);
 }
 
 // 7 resident blocks of 128: 72 registers, 28 warps per SM (spills, to L1).
@@ -578,6 +580,7 @@ static void launch_interp_block(int kb, DevBox *boxes, const Tile *tiles, int nt
 // spills) and 6 (80); 8 blocks (64 registers) is no faster.
 __global__ void __launch_bounds__(128, 7)
 k_be_mixed(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P, StepIn in) {
+    step_kernel_begin();
     const Tile tl = tiles[blockIdx.x];
     const DevBox &B = boxes[tl.box];
     Counts cnt;
@@ -589,6 +592,7 @@ k_be_mixed(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P
 
 __global__ void __launch_bounds__(kUpdateThreads)
 k_be_defer_mixed(DevBox *boxes, const __grid_constant__ DevParams P, StepIn in) {
+    step_kernel_begin();
     const DevBox &B = boxes[blockIdx.y];
     Counts cnt;
     for (int k = 0; k < kNumCounters; ++k) cnt.v[k] = 0;
@@ -611,16 +615,16 @@ void launch_update_be_mixed(int ilin, int nt, DevBox *boxes, const Tile *tiles, 
     if (ilin == 0 && blk_kb > 0 && n_blk_tiles > 0) {
         launch_interp_block(blk_kb, boxes, blk_tiles, n_blk_tiles, st);
     } else if (nt == 256) {
-        if (ilin == 1) k_interp_mixed<1, 256, false><<<ntiles, 256, 0, st>>>(boxes, tiles);
-        else if (tex) k_interp_mixed<0, 256, true><<<ntiles, 256, 0, st>>>(boxes, tiles);
-        else k_interp_mixed<0, 256, false><<<ntiles, 256, 0, st>>>(boxes, tiles);
+        if (ilin == 1) launch_step_kernel(k_interp_mixed<1, 256, false>, ntiles, 256, 0, st, boxes, tiles);
+        else if (tex) launch_step_kernel(k_interp_mixed<0, 256, true>, ntiles, 256, 0, st, boxes, tiles);
+        else launch_step_kernel(k_interp_mixed<0, 256, false>, ntiles, 256, 0, st, boxes, tiles);
     } else {
-        if (ilin == 1) k_interp_mixed<1, 128, false><<<ntiles, 128, 0, st>>>(boxes, tiles);
-        else if (tex) k_interp_mixed<0, 128, true><<<ntiles, 128, 0, st>>>(boxes, tiles);
-        else k_interp_mixed<0, 128, false><<<ntiles, 128, 0, st>>>(boxes, tiles);
+        if (ilin == 1) launch_step_kernel(k_interp_mixed<1, 128, false>, ntiles, 128, 0, st, boxes, tiles);
+        else if (tex) launch_step_kernel(k_interp_mixed<0, 128, true>, ntiles, 128, 0, st, boxes, tiles);
+        else launch_step_kernel(k_interp_mixed<0, 128, false>, ntiles, 128, 0, st, boxes, tiles);
     }
-    k_be_mixed<<<ntiles128, 128, 0, st>>>(boxes, tiles128, P, in);
-    k_be_defer_mixed<<<dim3(kDeferBlocks, nbox), kUpdateThreads, 0, st>>>(boxes, P, in);
+    launch_step_kernel(k_be_mixed, ntiles128, 128, 0, st, boxes, tiles128, P, in);
+    launch_step_kernel(k_be_defer_mixed, dim3(kDeferBlocks, nbox), kUpdateThreads, 0, st, boxes, P, in);
 }
 
 // Mixed payload from the stored state, for a coupling call whose dt differs
@@ -650,12 +654,10 @@ template <int V>
 static void depm(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P, cudaStream_t st,
                  int *overflow_list, bool dense) {
     constexpr int TX = kDepShape[V][0], TY = kDepShape[V][1], TZ = kDepShape[V][2];
-    cudaMemsetAsync(overflow_list, 0, sizeof(int), st);
-    k_deposit_tiled<TX, TY, TZ>
-        <<<ntiles, kDepositThreads, dep_smem_bytes(true, TX, TY, TZ), st>>>(boxes, tiles, P, overflow_list,
+    launch_step_kernel(k_deposit_tiled<TX, TY, TZ>, ntiles, kDepositThreads, dep_smem_bytes(true, TX, TY, TZ), st, boxes, tiles, P, overflow_list,
                                                                            dense ? 1 : 0);
     const int g = ntiles < kDenseBlocks ? ntiles : kDenseBlocks;
-    k_deposit_overflow32<TX, TY, TZ><<<g, kDepositThreads, 0, st>>>(boxes, tiles, P, overflow_list);
+    launch_step_kernel(k_deposit_overflow32<TX, TY, TZ>, g, kDepositThreads, 0, st, boxes, tiles, P, overflow_list);
 }
 
 template <int V>
@@ -679,10 +681,10 @@ void launch_deposit_mixed(int variant, DevBox *boxes, const Tile *tiles, int nti
     if (variant == 1) depm<1>(boxes, tiles, ntiles, P, st, overflow_list, dense);
     else if (variant == 2) depm<2>(boxes, tiles, ntiles, P, st, overflow_list, dense);
     else depm<0>(boxes, tiles, ntiles, P, st, overflow_list, dense);
-    k_fold<<<dim3(kFoldBlocks, nbox), 256, 0, st>>>(boxes);
+    launch_step_kernel(k_fold, dim3(kFoldBlocks, nbox), 256, 0, st, boxes, overflow_list);
     if (dense) {
-        k_cellsums32<<<dim3(kDenseBlocks, nbox), 256, 0, st>>>(boxes, P);
-        k_nodes_dense32<<<dim3(kDenseBlocks, nbox), 256, 0, st>>>(boxes);
+        launch_step_kernel(k_cellsums32, dim3(kDenseBlocks, nbox), 256, 0, st, boxes, P);
+        launch_step_kernel(k_nodes_dense32, dim3(kDenseBlocks, nbox), 256, 0, st, boxes);
     }
 }
 

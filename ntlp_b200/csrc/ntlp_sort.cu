@@ -24,6 +24,7 @@ namespace ntlp {
 __device__ __forceinline__ long long nbuckets(const DevBox &B) { return B.g.ncells + 2; }
 
 __global__ void k_scan_sums(DevBox *boxes, const Tile *tiles, long long *sums) {
+    step_kernel_begin();
     const Tile tl = tiles[blockIdx.x];
     const DevBox &B = boxes[tl.box];
     const long long nb = nbuckets(B);
@@ -45,6 +46,7 @@ __global__ void k_scan_sums(DevBox *boxes, const Tile *tiles, long long *sums) {
 
 // one block per box: exclusive scan of the box's tile sums, in place
 __global__ void k_scan_offsets(const int *box_first_tile, long long *sums) {
+    step_kernel_begin();
     const int b = blockIdx.x;
     const int a = box_first_tile[b], e = box_first_tile[b + 1];
     __shared__ long long carry;
@@ -82,6 +84,7 @@ __global__ void k_scan_offsets(const int *box_first_tile, long long *sums) {
 // local exclusive scan of each tile plus its offset; counts are cleared (the
 // array becomes the scatter cursor)
 __global__ void k_scan_local(DevBox *boxes, const Tile *tiles, const long long *offs) {
+    step_kernel_begin();
     const Tile tl = tiles[blockIdx.x];
     const DevBox &B = boxes[tl.box];
     const long long nb = nbuckets(B);
@@ -125,6 +128,7 @@ __global__ void k_scan_local(DevBox *boxes, const Tile *tiles, const long long *
 
 // ---- scatter ---------------------------------------------------------------
 __global__ void k_scatter(DevBox *boxes, const Tile *tiles) {
+    step_kernel_begin();
     const Tile tl = tiles[blockIdx.x];
     const DevBox &B = boxes[tl.box];
     const int t = tl.start + threadIdx.x;
@@ -149,6 +153,7 @@ __global__ void k_scatter(DevBox *boxes, const Tile *tiles) {
 // global memory, one thread per cell: the whole sort of 2 M droplets at 31 per
 // cell took 0.71 ms, it takes 0.089 (16.8 M at one per cell: 0.44 -> 0.41).
 __global__ void __launch_bounds__(kUpdateThreads) k_cellrank(DevBox *boxes, const Tile *tiles) {
+    step_kernel_begin();
     __shared__ int s_lid[kUpdateThreads];
     const Tile tl = tiles[blockIdx.x];
     const DevBox &B = boxes[tl.box];
@@ -185,16 +190,17 @@ __global__ void __launch_bounds__(kUpdateThreads) k_cellrank(DevBox *boxes, cons
 }
 
 void launch_sort(DevBox *boxes, const SortPlan &plan, cudaStream_t st) {
-    k_scan_sums<<<plan.n_cell_tiles, 256, 0, st>>>(boxes, plan.cell_tiles, plan.tile_sums);
-    k_scan_offsets<<<plan.nbox, 1024, 0, st>>>(plan.box_first_tile, plan.tile_sums);
-    k_scan_local<<<plan.n_cell_tiles, kCellThreads, 0, st>>>(boxes, plan.cell_tiles, plan.tile_sums);
-    k_scatter<<<plan.n_drop_tiles, kUpdateThreads, 0, st>>>(boxes, plan.drop_tiles);
+    launch_step_kernel(k_scan_sums, plan.n_cell_tiles, 256, 0, st, boxes, plan.cell_tiles, plan.tile_sums);
+    launch_step_kernel(k_scan_offsets, plan.nbox, 1024, 0, st, plan.box_first_tile, plan.tile_sums);
+    launch_step_kernel(k_scan_local, plan.n_cell_tiles, kCellThreads, 0, st, boxes, plan.cell_tiles, plan.tile_sums);
+    launch_step_kernel(k_scatter, plan.n_drop_tiles, kUpdateThreads, 0, st, boxes, plan.drop_tiles);
     if (plan.n_drop_tiles > 0)
-        k_cellrank<<<plan.n_drop_tiles, kUpdateThreads, 0, st>>>(boxes, plan.drop_tiles);
+        launch_step_kernel(k_cellrank, plan.n_drop_tiles, kUpdateThreads, 0, st, boxes, plan.drop_tiles);
 }
 
 // ---- finish: flip buffers, count survivors ---------------------------------
 __global__ void k_finish(DevBox *boxes, int nbox) {
+    step_kernel_begin();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nbox) return;
     DevBox &B = boxes[b];
@@ -206,10 +212,11 @@ __global__ void k_finish(DevBox *boxes, int nbox) {
 }
 
 void launch_finish(DevBox *boxes, int nbox, cudaStream_t st) {
-    k_finish<<<(nbox + 127) / 128, 128, 0, st>>>(boxes, nbox);
+    launch_step_kernel(k_finish, (nbox + 127) / 128, 128, 0, st, boxes, nbox);
 }
 
 __global__ void k_reset_step(DevBox *boxes, int nbox) {
+    step_kernel_begin();
     const DevBox &B = boxes[blockIdx.x];
     const int nz1 = B.g.nnz + 1;
     for (int i = threadIdx.x; i < kNumCounters; i += blockDim.x) B.counters[i] = 0;
@@ -223,7 +230,7 @@ __global__ void k_reset_step(DevBox *boxes, int nbox) {
 }
 
 void launch_reset_step(DevBox *boxes, int nbox, cudaStream_t st) {
-    k_reset_step<<<nbox, 256, 0, st>>>(boxes, nbox);
+    launch_step_kernel(k_reset_step, nbox, 256, 0, st, boxes, nbox);
 }
 
 // keys of a freshly uploaded state (held in st[1-cur], list order)
@@ -338,6 +345,7 @@ __device__ __forceinline__ void fill_tile(const FieldSrc &s, const DevGrid &g, c
 
 template <bool MIXED>
 __global__ void __launch_bounds__(256) k_fill_flow(const __grid_constant__ DevBox B, FieldSrc s) {
+    step_kernel_begin();
     __shared__ double tile[5][32][33];
     if constexpr (MIXED) {
         const bool first = blockIdx.x + blockIdx.y + blockIdx.z == 0 && threadIdx.x + threadIdx.y == 0;
@@ -372,8 +380,8 @@ void launch_fill_fields(const DevBox &B, const FieldSrc &s, bool flow, cudaStrea
     const DevGrid &g = B.g;
     if (flow) {
         const dim3 grid((g.nnx + 5 + 31) / 32, (g.nnz + 2 + 31) / 32, g.nny + 5), block(32, 8);
-        if (B.f4) k_fill_flow<true><<<grid, block, 0, st>>>(B, s);
-        else k_fill_flow<false><<<grid, block, 0, st>>>(B, s);
+        if (B.f4) launch_step_kernel(k_fill_flow<true>, grid, block, 0, st, B, s);
+        else launch_step_kernel(k_fill_flow<false>, grid, block, 0, st, B, s);
         return;
     }
     const long long n = (long long)g.nz2 * g.ny5 * g.nx5;

@@ -1,0 +1,35 @@
+"""Mixed deposition tiles above their stage's capacity (768 droplets): taken in
+slabs of levels, or a level from global memory, against the per-cell sums that
+boxes of large capacity use.  The sources are the same bits."""
+import numpy as np
+import pytest
+
+from conftest import cuda_available
+from helpers import bitwise_equal, small_case
+from ntlp_b200 import abi
+from ntlp_b200 import generator as gen
+
+
+@pytest.mark.parametrize("grid_n,n", [
+    ((9, 9, 70), 30_000),     # slabs of many levels, ragged tiles in every direction
+    ((5, 3, 40), 9_000),      # about 9 a cell
+    ((4, 5, 33), 14_000),     # slabs of a level or two
+    ((2, 2, 3), 2_500),       # one level's cells exceed the stage
+])
+@pytest.mark.gpu
+@pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")
+def test_slabs_match_cell_sums(grid_n, n):
+    import ntlp_b200
+    params = dict(gen.default_params(icase=0), precision=abi.NTLP_PREC_MIXED)
+    case = small_case(params=params, n=n, grid_n=grid_n)
+    ncells = (grid_n[0] + 1) * (grid_n[1] + 1) * (grid_n[2] + 1)
+    out = []
+    for cap in (n, max(n, 16 * ncells)):
+        s = ntlp_b200.DropletStep(case.grid, params, capacity=cap)
+        s.set_fields_ext(case.ext())
+        s.set_droplets(case.droplets)
+        s.particle_update_BE(case.dt, 1)
+        out.append([np.asarray(x).copy() for x in s.particle_coupling_update(case.dt)])
+        s.close()
+    for q in range(6):
+        assert bitwise_equal(out[0][q], out[1][q]), q
