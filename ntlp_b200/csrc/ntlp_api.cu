@@ -531,6 +531,25 @@ struct Src6 {
     double *p[6];
 };
 
+// the six source arrays of a box into arrays on the device (dst NULL: not
+// wanted): one launch, where six copies cost more to issue than to run in a
+// small box
+__global__ void __launch_bounds__(256) k_copy_sources(Src6 src, Src6 dst, long long n) {
+    const double *__restrict__ s = src.p[blockIdx.y];
+    double *__restrict__ d = dst.p[blockIdx.y];
+    if (d == nullptr) return;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * stride) {
+        double v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (i + k * stride < n) v[k] = __ldcs(s + i + k * stride);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (i + k * stride < n) __stcs(d + i + k * stride, v[k]);
+    }
+}
+
 __global__ void k_iota(int *a, int n) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) a[t] = t;
@@ -1319,10 +1338,18 @@ int sources_out(ntlp_ctx *c, int b, int32_t layout, double *const host[6]) {
         if (any) CK(cudaStreamSynchronize(c->stream));
         return NTLP_OK;
     }
+    Src6 from{}, here{};   // arrays on this device: column layout, copied in one launch
+    bool direct = false;
     for (int q = 0; q < 6; ++q) {
         if (!host[q]) continue;
         any = true;
         const double *src = B.src[q];
+        if (layout == NTLP_LAYOUT_COLUMN && on_device(c, host[q], 8)) {
+            from.p[q] = B.src[q];
+            here.p[q] = host[q];
+            direct = true;
+            continue;
+        }
         if (layout == NTLP_LAYOUT_FLOW) {
             dim3 grid((g.nnx + 31) / 32, (g.nz2 + 31) / 32, g.nny);
             k_col_to_flow<<<grid, dim3(32, 8), 0, c->stream>>>(src, c->bh[b].staging, g.nnx, g.nny, g.nz2);
@@ -1331,6 +1358,11 @@ int sources_out(ntlp_ctx *c, int b, int32_t layout, double *const host[6]) {
         }
         CK(cudaMemcpyAsync(host[q], src, nn * 8, cudaMemcpyDefault, c->stream));
         if (layout == NTLP_LAYOUT_FLOW) CK(cudaStreamSynchronize(c->stream));
+    }
+    if (direct) {
+        const long long blocks = std::min<long long>(((long long)nn + 1023) / 1024, 148 * 8);
+        k_copy_sources<<<dim3((unsigned)blocks, 6), 256, 0, c->stream>>>(from, here, (long long)nn);
+        c->launches += 1;
     }
     if (any) CK(cudaStreamSynchronize(c->stream));
     CK(cudaGetLastError());

@@ -361,8 +361,12 @@ __global__ void k_fold(DevBox *boxes, int *overflow_list) {
     const long long na = (long long)ya * g.nnx * g.nz2;                       // iy <= 2, every ix
     const long long nb = g.nny > 2 ? (long long)xb * (g.nny - 2) * g.nz2 : 0;  // ix <= 2, iy >= 3
     const long long per = img_count(g);
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < na + nb;
-         idx += (long long)gridDim.x * blockDim.x) {
+    // a thread per (quantity, node): one node's six values in turn made a chain
+    // of loads, 14 us even in a 32^3 box
+    for (long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x; at < 6 * (na + nb);
+         at += (long long)gridDim.x * blockDim.x) {
+        const int q = (int)(at / (na + nb));
+        const long long idx = at - q * (na + nb);
         int ix, iy, iz;
         if (idx < na) {
             iz = (int)(idx % g.nz2);
@@ -375,17 +379,15 @@ __global__ void k_fold(DevBox *boxes, int *overflow_list) {
             ix = 1 + (int)(r / ((long long)g.nz2 * (g.nny - 2)));
         }
         const long long node = (long long)iz + (long long)g.nz2 * ((long long)(iy - 1) + (long long)g.sny * (ix - 1));
-        for (int q = 0; q < 6; ++q) {
-            const double *I = B.img + q * per;
-            double out = B.src[q][node];
-            if (ix <= 2) out = out + I[img_index(g, ix + g.nnx, iy, iz)];
-            if (iy <= 2) {
-                double b0 = I[img_index(g, ix, iy + g.nny, iz)];
-                if (ix <= 2) b0 = b0 + I[img_index(g, ix + g.nnx, iy + g.nny, iz)];
-                out = out + b0;
-            }
-            B.src[q][node] = out;
+        const double *I = B.img + q * per;
+        double out = B.src[q][node];
+        if (ix <= 2) out = out + I[img_index(g, ix + g.nnx, iy, iz)];
+        if (iy <= 2) {
+            double b0 = I[img_index(g, ix, iy + g.nny, iz)];
+            if (ix <= 2) b0 = b0 + I[img_index(g, ix + g.nnx, iy + g.nny, iz)];
+            out = out + b0;
         }
+        B.src[q][node] = out;
     }
 }
 
