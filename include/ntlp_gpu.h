@@ -206,9 +206,11 @@ int ntlp_stream_priority(ntlp_ctx *ctx, int32_t priority);
  * kernel (stencil from global memory; the same results, bit for bit), 1
  * back to the staged one, -1 only queries; 4, 8, 16 or 32 sets the block
  * height in cells (blocks are 4 x 4 x height cells; the context picks one
- * for about 256 droplets a block, ntlp_autotune tries half and twice that)
- * and switches staging on.
- * Returns the block height in cells (0: per-droplet kernel) or an error
+ * from its droplets per cell, ntlp_autotune tries half and twice that)
+ * and switches staging on.  Until a call sets it, the context stages only
+ * where that is the faster of the two: in boxes of a million droplets or
+ * more with 0.75 to 40 of them per cell.
+ * Returns the block height in cells (0: switched off) or an error
  * code (< 0).  The results do not depend on it.  No counterpart in the
  * reference.                                                              */
 int ntlp_interp_staging(ntlp_ctx *ctx, int32_t enable);

@@ -138,6 +138,7 @@ struct ntlp_ctx {
     // tiles; blk_kb = 0 when the tensor maps could not be made
     int blk_kb = 0;
     bool blk_on = true;
+    bool blk_auto = true, blk_pays = true;   // until ntlp_interp_staging sets it: staged where it pays
     Tile *blk_tiles_d = nullptr;
     int n_blk_tiles = 0;
     int blk_tile_cap = 0;   // tiles blk_tiles_d holds (the smallest block height the tuner tries)
@@ -825,7 +826,7 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
             return bail(fail(c, NTLP_ERR_CUDA, "initialising box %d failed", b));
     }
     // staged interpolation (mixed, 6th order): one block height for the
-    // context, from its droplets per cell
+    // context, from its droplets per cell, and whether it is used at all
     if (mixed && params->ilin == 0) {
         double caps_sum = 0.0, cells = 0.0;
         for (int b = 0; b < nbox; ++b) {
@@ -833,6 +834,7 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
             cells += (double)c->box[b].g.ncells;
         }
         c->blk_kb = interp_block_kb(caps_sum / cells);
+        c->blk_pays = interp_staged_pays(caps_sum / cells, caps_sum);
         for (int b = 0; b < nbox && c->blk_kb; ++b)
             if (!encode_f4_map(c->box[b], c->blk_kb)) c->blk_kb = 0;
         for (int b = 0; b < nbox; ++b) c->box[b].blk_kb = c->blk_kb;
@@ -1206,6 +1208,11 @@ int deposit_launches(const ntlp_ctx *c) {
     return c->any_dense ? 5 : 3;   // tiles, overflow, fold (+ cell sums, dense nodes)
 }
 
+// whether the step interpolates over staged blocks
+bool staged_interp(const ntlp_ctx *c) {
+    return c->blk_on && c->blk_kb > 0 && (!c->blk_auto || c->blk_pays);
+}
+
 // launch the kernels of one step (no synchronisation; graph-capturable)
 int launch_step(ntlp_ctx *c, int kind, int istage, double dt, int32_t it, bool with_deposit) {
     const int nt = kNtValues[c->nt_variant];
@@ -1223,7 +1230,7 @@ int launch_step(ntlp_ctx *c, int kind, int istage, double dt, int32_t it, bool w
         if (c->params.precision == NTLP_PREC_MIXED)
             launch_update_be_mixed(c->params.ilin, nt, c->box_d, c->drop_tiles_d[c->nt_variant],
                                    c->n_drop_tiles[c->nt_variant], c->drop_tiles_d[0], c->n_drop_tiles[0], c->nbox,
-                                   c->dp, in, c->stream, c->tex_all, c->blk_on ? c->blk_kb : 0, c->blk_tiles_d,
+                                   c->dp, in, c->stream, c->tex_all, staged_interp(c) ? c->blk_kb : 0, c->blk_tiles_d,
                                    c->n_blk_tiles);
         else
             launch_update_be64(c->params.ilin, nt, c->box_d, c->drop_tiles_d[c->nt_variant],
@@ -1570,10 +1577,12 @@ int ntlp_interp_staging(ntlp_ctx *c, int32_t enable) {
     if (!c) return NTLP_ERR_ARG;
     if (enable == 0 || enable == 1) {
         c->blk_on = enable == 1;
+        c->blk_auto = false;
     } else if (enable >= 2) {
         int rc = set_blk_kb(c, enable);
         if (rc) return rc;
         c->blk_on = true;
+        c->blk_auto = false;
     } else if (enable != -1) {
         return fail(c, NTLP_ERR_ARG, "staging switch %d", enable);
     }
@@ -1782,7 +1791,7 @@ int ntlp_flux(ntlp_ctx *c, double *pflux, double *pmassflux, double *penegflux) 
 // instantiate it, unless the one held matches dt, nsteps and the variants
 static int build_graph(ntlp_ctx *c, double dt, int32_t it, int32_t nsteps) {
     if (c->gexec && c->g_dt == dt && c->g_nsteps == nsteps && c->g_dep == c->dep_variant &&
-        c->g_nt == c->nt_variant && c->g_blk == c->blk_on && c->g_kb == c->blk_kb)
+        c->g_nt == c->nt_variant && c->g_blk == staged_interp(c) && c->g_kb == c->blk_kb)
         return NTLP_OK;
     if (c->gexec) {
         cudaGraphExecDestroy(c->gexec);
@@ -1814,7 +1823,7 @@ static int build_graph(ntlp_ctx *c, double dt, int32_t it, int32_t nsteps) {
     c->g_nsteps = nsteps;
     c->g_dep = c->dep_variant;
     c->g_nt = c->nt_variant;
-    c->g_blk = c->blk_on;
+    c->g_blk = staged_interp(c);
     c->g_kb = c->blk_kb;
     return NTLP_OK;
 }
@@ -1923,6 +1932,8 @@ int ntlp_autotune(ntlp_ctx *c, double dt, int32_t it, int32_t steps, int32_t cho
     // it and twice it (within 4..32 and the tile table)
     if (!rc && c->blk_kb > 0 && c->blk_on) {
         const int kb0 = c->blk_kb;
+        const bool automatic = c->blk_auto;
+        c->blk_auto = false;
         int best_kb = kb0;
         double best_ms = local[kDepVariants + best_nt];
         const int cand[2] = {kb0 / 2, kb0 * 2};
@@ -1940,6 +1951,7 @@ int ntlp_autotune(ntlp_ctx *c, double dt, int32_t it, int32_t steps, int32_t cho
             }
         }
         if (!rc) rc = set_blk_kb(c, best_kb);
+        if (best_kb == kb0) c->blk_auto = automatic;
     }
     c->prof = prof;
     cudaEventDestroy(a);

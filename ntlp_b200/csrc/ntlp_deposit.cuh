@@ -471,6 +471,11 @@ k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams 
     bool staged = images || ((x0 > 2) && (y0 > 2));
     if (staged) {
         const int total = tile_columns<TX, TY, TZ>(B, x0, y0, z0, s_cs, s_off);
+        if (total == 0) {
+            const double zero[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            if (valid) store_node(B, ix, iy, iz, zero);
+            return;
+        }
         staged = total <= CAP;
         if (staged) {
             // two droplets per pass: their loads are in flight together
@@ -574,6 +579,11 @@ k_deposit_tiled(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevPar
     const int ix = x0 + lx, iy = y0 + ly, iz = z0 + lz;
     const bool valid = ix <= g.dnx && iy <= g.dny && iz <= g.nnz + 1;
     const int total = tile_columns<kDepTX, kDepTY, kDepTZ>(B, x0, y0, z0, s_cs, s_off);
+    if (total == 0) {
+        const double zero[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        if (valid) store_node(B, ix, iy, iz, zero);
+        return;
+    }
     if (total > CAP) {
         // above the stage capacity: k_deposit_overflow32, which has the
         // registers of the global path

@@ -95,15 +95,21 @@ constexpr int kBlockThreads = 160;   // threads of a cell-block interpolation CT
 constexpr int kOobBlockTiles = 8;    // tiles per box over the out-of-range bucket
 int interp_block_smem(int kb);       // dynamic shared memory of a cell-block CTA
 void prepare_interp_block();         // kernel attributes, once per device
-// cells per block in z for a droplet density (droplets per cell): about 256
-// droplets per block, one of 4, 8, 16, 32.  Measured at one droplet per cell
-// (16.8 M droplets, 256^3, update phase with 160 threads per CTA): 16 cells
-// 6.06 ms, 8 cells 6.30 ms, 32 cells 6.24 ms; 16 cells with 192, 256 or 288
-// threads 6.26, 6.43, 6.12 ms.
-inline int interp_block_kb(double density) {
-    const double want = 256.0 / (kBlkX * kBlkY * (density > 1e-9 ? density : 1e-9));
-    int kb = 4 * (int)(want / 4.0 + 0.5);
-    return kb < 4 ? 4 : (kb > 32 ? 32 : (kb > 16 ? 32 : (kb > 8 ? 16 : kb)));
+// Cells per block in z for a droplet density (droplets per cell).  Update phase
+// with 8 / 16 / 32 cells: 16.7 M droplets at 0.98 per cell 5.95 / 5.61 / 6.0 ms, 4 M at
+// 1.9 1.21 / 1.18 ms, 67 M at 2 (4 where there are any) 18.8 / 18.2 ms; 1 M at
+// 3.6 with 4 / 8 / 16: 0.331 / 0.326 / 0.341 ms, 2 M at 29 0.624 / 0.649 / 0.786 ms.
+inline int interp_block_kb(double density) { return density < 3.0 ? 16 : (density < 6.0 ? 8 : 4); }
+// Whether the staged blocks beat the per-droplet kernel (the same bits): a block
+// stages 3.2 KB of fields per cell column and 16 levels whether it holds
+// droplets or not, and its CTAs take turns of latency that a small box cannot
+// overlap.  Update phase, per droplet against staged: 0.063 against 0.143 ms (10,000
+// droplets, 0.005 per cell), 0.275 against 0.341 (500,000, 0.23), 3.27 against
+// 3.53 (8 M, 0.47), 0.121 against 0.126 (250,000, 0.91), 0.190 against 0.188 (500,000,
+// 1.8); 0.737 against 0.732 (2 M, 0.93), 5.83 against 5.61 (16.7 M, 0.98), 1.28 against
+// 1.18 (4 M, 1.9), 0.637 against 0.624 (2 M, 29); 0.660 against 0.686 (2 M, 56).
+inline bool interp_staged_pays(double density, double droplets) {
+    return density >= 0.75 && density < 40.0 && droplets >= 1e6;
 }
 inline long long interp_block_count(int kb, int nnx, int nny, int nnz) {
     return (long long)((nnx + kBlkX) / kBlkX) * ((nny + kBlkY) / kBlkY) * ((nnz + kb) / kb);

@@ -121,3 +121,27 @@ def test_staged_interpolation_in_a_batch():
             assert bitwise_equal(da[k], db[k]), k
         for q in range(6):
             assert bitwise_equal(np.asarray(sa[q]), np.asarray(sb[q])), q
+
+
+@pytest.mark.parametrize("edge,n,height", [
+    (20, 2_000, 16),            # small: per droplet unless asked for
+    (40, 1_000_000, 4),         # dense enough and large enough: staged
+    (24, 1_000_000, 4),         # 64 per cell: per droplet
+])
+def test_default_choice_gives_the_same_bits(edge, n, height):
+    import ntlp_b200
+    params = dict(gen.default_params(ilin=0), precision=abi.NTLP_PREC_MIXED)
+    case = small_case(params=params, n=n, grid_n=(edge, edge, edge))
+    out = []
+    for setting in (None, 1, 0):
+        s = ntlp_b200.DropletStep(case.grid, params, capacity=n)
+        assert s.interp_staging(-1) == height
+        if setting is not None:
+            assert s.interp_staging(setting) == (height if setting else 0)
+        s.set_fields_ext(case.ext())
+        s.set_droplets(case.droplets)
+        s.particle_update_BE(case.dt, 1)
+        out.append(s.get_droplets())
+        s.close()
+    for k in STATE_KEYS:
+        assert bitwise_equal(out[0][k], out[1][k]) and bitwise_equal(out[0][k], out[2][k]), k
