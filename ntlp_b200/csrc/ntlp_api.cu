@@ -320,7 +320,7 @@ void carve_box(Carver &cv, BoxHost &h, DevBox &B, bool mixed) {
     B.img = nullptr;
     if (g.periodic) cv.take(&B.img, 6 * (size_t)img_count(g));
     if (mixed) {
-        for (int q = 0; q < P32_N; ++q) cv.take(&B.pay32.f[q], n);
+        cv.take(&B.pay32.p, kPay32Words * n);
         B.cellsum = nullptr;
         if ((long long)h.cap >= (long long)kDenseRatio * g.ncells) cv.take(&B.cellsum, (size_t)g.ncells * 48);
     } else {

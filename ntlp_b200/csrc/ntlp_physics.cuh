@@ -690,15 +690,16 @@ __device__ __forceinline__ void write_payload_mixed(const DevBox &B, const DevPa
     // nuf cancel): the same quantities without their divides
     const float partmass = (float)m_s + volp * rhow;
     const float H0 = rhow * irhoa * pi2 * 2.0f * (rf * rf) * (float)radrhs;
-    float *const *f = B.pay32.f;
-    f[P32_FX][t] = (float)((x[0] - g.dx * (double)(ipt + g.ioff - 1)) * g.rdx);
-    f[P32_FY][t] = (float)((x[1] - g.dy * (double)(jpt + g.joff - 1)) * g.rdy);
-    f[P32_FZ][t] = (float)(x[2] - g.zz[kpt]) / (float)g.dzu[kpt + 1];
-    for (int a = 0; a < 3; ++a) f[P32_DV0 + a][t] = partmass * irhoa * (vrhs[a] - p.f_g[a]) + H0 * (float)v[a];
-    f[P32_T0][t] = (float)Tprhs_s * volp * p.f_rhow_cc * irhoa;
-    f[P32_H0][t] = H0;
-    f[P32_E][t] = H0 * p.f_cpv_cpa * (float)(Tf - Tp);
-    f[P32_FAC][t] = (float)((double)mult / (g.dx * g.dy * g.dzu[kpt + 1]));
+    float f[P32_N];
+    f[P32_FX] = (float)((x[0] - g.dx * (double)(ipt + g.ioff - 1)) * g.rdx);
+    f[P32_FY] = (float)((x[1] - g.dy * (double)(jpt + g.joff - 1)) * g.rdy);
+    f[P32_FZ] = (float)(x[2] - g.zz[kpt]) / (float)g.dzu[kpt + 1];
+    for (int a = 0; a < 3; ++a) f[P32_DV0 + a] = partmass * irhoa * (vrhs[a] - p.f_g[a]) + H0 * (float)v[a];
+    f[P32_T0] = (float)Tprhs_s * volp * p.f_rhow_cc * irhoa;
+    f[P32_H0] = H0;
+    f[P32_E] = H0 * p.f_cpv_cpa * (float)(Tf - Tp);
+    f[P32_FAC] = (float)((double)mult / (g.dx * g.dy * g.dzu[kpt + 1]));
+    store_payload32(B.pay32, t, f);
 }
 
 // Backward-Euler drag update of the velocity (particles.f90:3083-3100);
