@@ -105,6 +105,7 @@ struct ntlp_ctx {
     void *small_arena = nullptr;
     SortPlan plan{};
     int dep_variant = 0, nt_variant = 0;
+    int dep64_cap = 0;                // FP64 deposition: stage capacity (deposit64_cap)
     long long *counters_h = nullptr;   // pinned [nbox][kNumCounters]
     int *err_h = nullptr;              // pinned [nbox] device error words
     // device-timed steps (ntlp_step_timed): an event pair per slot
@@ -325,9 +326,7 @@ void carve_box(Carver &cv, BoxHost &h, DevBox &B, bool mixed) {
         if ((long long)h.cap >= (long long)kDenseRatio * g.ncells) cv.take(&B.cellsum, (size_t)g.ncells * 48);
     } else {
         B.cellsum = nullptr;
-        for (int a = 0; a < 3; ++a) { cv.take(&B.pay.D[a], n); cv.take(&B.pay.V[a], n); }
-        cv.take(&B.pay.T0, n); cv.take(&B.pay.H0, n); cv.take(&B.pay.E1, n); cv.take(&B.pay.E2, n);
-        cv.take(&B.pay.mult, n);
+        cv.take(&B.pay.p, kPay64Words * n);
     }
     cv.take(&B.n_alive, 1);
     cv.take(&B.perm, n);
@@ -839,6 +838,12 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
             if (!encode_f4_map(c->box[b], c->blk_kb)) c->blk_kb = 0;
         for (int b = 0; b < nbox; ++b) c->box[b].blk_kb = c->blk_kb;
     }
+    if (!mixed) {
+        double density = 0.0;   // of the fullest box
+        for (int b = 0; b < nbox; ++b)
+            density = std::max(density, (double)c->bh[b].cap / (double)c->box[b].g.ncells);
+        c->dep64_cap = deposit64_cap(density);
+    }
     // tiles: droplets (128 and 256 per tile), cells (scan tiles), deposition
     // (3 shapes), interpolation cell blocks
     std::vector<Tile> dt[kNtVariants], ct, dpt[kDepVariants], bt;
@@ -1204,7 +1209,7 @@ int droplets_download(ntlp_ctx *c, int b, ntlp_droplets *d) {
 // kernels of one deposition: the tiles, plus the two cell-sum kernels when
 // a mixed box is dense
 int deposit_launches(const ntlp_ctx *c) {
-    if (c->params.precision != NTLP_PREC_MIXED) return 2;   // tiles, fold
+    if (c->params.precision != NTLP_PREC_MIXED) return 3;   // tiles, overflow, fold
     return c->any_dense ? 5 : 3;   // tiles, overflow, fold (+ cell sums, dense nodes)
 }
 
@@ -1254,7 +1259,8 @@ int launch_step(ntlp_ctx *c, int kind, int istage, double dt, int32_t it, bool w
             launch_deposit_mixed(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
                                  c->any_dense, c->overflow_list_d);
         else
-            launch_deposit64(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox);
+            launch_deposit64(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
+                             c->dep64_cap, c->overflow_list_d);
         phase_end(c, PH_DEPOSIT, e0);
         c->launches += deposit_launches(c);
     }
@@ -1442,7 +1448,8 @@ int launch_coupling(ntlp_ctx *c, double dt) {
         launch_deposit_mixed(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
                              c->any_dense, c->overflow_list_d);
     else
-        launch_deposit64(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox);
+        launch_deposit64(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
+                             c->dep64_cap, c->overflow_list_d);
     phase_end(c, PH_DEPOSIT, e0);
     c->launches += deposit_launches(c);
     CK(cudaGetLastError());

@@ -35,7 +35,6 @@
 namespace ntlp {
 namespace {
 
-constexpr int kDepCap64 = 640;                                    // droplets staged per tile (FP64)
 constexpr int kDepCapMixed = 768;                                 // droplets staged per tile (mixed)
 // mixed stage: the six source factors of a droplet in FP64 (signs applied,
 // converted once per droplet, not once per node), then fx, fy, fz, mult/dV
@@ -133,10 +132,12 @@ __device__ __forceinline__ void merge_ranges(const DevBox &B, const DevParams &p
         if (pos[best] < end[best]) head[best] = O.lid[B.perm[pos[best]]];
         DropVals d;
         const int t = B.perm[at];
-        const DevPayload &P = B.pay;
+        double v[P64_N];
+        int lid, key;
+        load_payload64(B.pay, t, v, lid, key);
         d.x1 = O.x[0][t]; d.x2 = O.x[1][t]; d.x3 = O.x[2][t];
-        for (int a = 0; a < 3; ++a) { d.D[a] = P.D[a][t]; d.V[a] = P.V[a][t]; }
-        d.T0 = P.T0[t]; d.H0 = P.H0[t]; d.E1 = P.E1[t]; d.E2 = P.E2[t]; d.mult = P.mult[t];
+        for (int a = 0; a < 3; ++a) { d.D[a] = v[P64_D + a]; d.V[a] = v[P64_V + a]; }
+        d.T0 = v[P64_T0]; d.H0 = v[P64_H0]; d.E1 = v[P64_E1]; d.E2 = v[P64_E2]; d.mult = v[P64_MULT];
         contribute64(g, p, d, kpt, xv, yv, zv, acc);
     }
 }
@@ -162,19 +163,22 @@ __device__ __forceinline__ bool plain_num(double v) {
     return v == 0.0 || (hi >= ((1023u - 600u) << 20) && hi < ((1023u + 900u) << 20));
 }
 
-// stage of the FP64 tiles: droplet factors and trilinear weights, one array
-// of kDepCap64 per value
-enum { V64_D = 0, V64_V = 3, V64_T0 = 6, V64_H0, V64_E1, V64_E2, V64_MULT, V64_WX, V64_WY = V64_WX + 2,
-       V64_WZ = V64_WY + 2, V64_N = V64_WZ + 2 };
+// Stage of an FP64 tile: lid, slot and trilinear weights of up to `cap`
+// droplets, one array per value.  The factors stay in the payload, whose three
+// 32-byte words a node reads where it needs them (L1, mostly): staged as
+// well, they took 140 bytes a droplet and held the SM at two CTAs of 128
+// registers (16.8 M droplets: 4.69 ms, against 4.15 at three CTAs of 80, and
+// 4.66 at four of 64).
+enum { V64_WX = 0, V64_WY = 2, V64_WZ = 4, V64_N = 6 };
+constexpr int kStage64 = V64_N * 8 + 2 * 4;   // bytes per droplet
 
 // One node from the stage: its cells' lists (run[c]: first stage position, end
 // << 16; c = i<<2 | j<<1 | k) merged by lid.  dV, rdV: cell volume of the
 // droplet's cell and its reciprocal, for k = 0 and 1.
-template <bool FAST>
-__device__ __forceinline__ void merge_staged64(const DevParams &p, const int *s_lid, const double *s_v,
+template <bool FAST, int CAP>
+__device__ __forceinline__ void merge_staged64(const DevBox &B, const DevParams &p, const int *s_lid, const int *s_t, const double *s_w,
                                                int (&run)[8], const double dV[2], const double rdV[2],
                                                double acc[6]) {
-    constexpr int CAP = kDepCap64;
     constexpr int kNone = 0x7fffffff;   // no lid is this large
     int head[8];
 #pragma unroll
@@ -194,27 +198,30 @@ __device__ __forceinline__ void merge_staged64(const DevParams &p, const int *s_
 #pragma unroll
         for (int c = 0; c < 8; ++c)
             if (c == o) { head[c] = next; run[c] = sel + 1; }
-        const double *v = s_v + at;
+        const double *w = s_w + at;
         const double d = (o & 1) ? dV[1] : dV[0], y = (o & 1) ? rdV[1] : rdV[0];
-        const double wtx = v[(V64_WX + (o >> 2)) * CAP];
-        const double wty = v[(V64_WY + ((o >> 1) & 1)) * CAP];
-        const double wtz = v[(V64_WZ + (o & 1)) * CAP];
+        const double wtx = w[(V64_WX + (o >> 2)) * CAP];
+        const double wty = w[(V64_WY + ((o >> 1) & 1)) * CAP];
+        const double wtz = w[(V64_WZ + (o & 1)) * CAP];
         const double wtt = wtx * wty * wtz;
-        const double mult = v[V64_MULT * CAP];
+        double v[P64_N];
+        int lid, key;
+        load_payload64(B.pay, s_t[at], v, lid, key);
+        const double mult = v[P64_MULT];
         auto term = [&](int q) {
-            const double a = v[q * CAP] * wtt;
+            const double a = v[q] * wtt;
             return (FAST ? div_by(a, d, y) : a / d) * mult;
         };
         if (p.icouple == 1) {
             for (int a = 0; a < 3; ++a) {
-                acc[a] = acc[a] - term(V64_D + a);
-                acc[a] = acc[a] - term(V64_V + a);
+                acc[a] = acc[a] - term(P64_D + a);
+                acc[a] = acc[a] - term(P64_V + a);
             }
         }
-        if (p.iTcouple == 1) acc[3] = acc[3] - term(V64_T0);
+        if (p.iTcouple == 1) acc[3] = acc[3] - term(P64_T0);
         if (p.iHcouple == 1) {
-            acc[4] = acc[4] - term(V64_H0);
-            acc[5] = acc[5] - term(V64_E1) + term(V64_E2);
+            acc[4] = acc[4] - term(P64_H0);
+            acc[5] = acc[5] - term(P64_E1) + term(P64_E2);
         }
     }
 }
@@ -403,7 +410,7 @@ __global__ void k_fold(DevBox *boxes, int *overflow_list) {
 
 // shared memory of a tile shape (TX x TY x TZ nodes)
 __host__ __device__ constexpr int dep_smem_bytes(bool mixed, int TX, int TY, int TZ) {
-    return (mixed ? kDepCapMixed * (kStageD * 8 + kStageF * 4) : kDepCap64 * (4 + V64_N * 8)) +
+    return (mixed ? kDepCapMixed * (kStageD * 8 + kStageF * 4) : 0) +
            (TX + 1) * (TY + 1) * (TZ + 2) * 4 + (TX + 1) * (TY + 1) * 4 + 16;
 }
 
@@ -452,19 +459,20 @@ __device__ __forceinline__ int tile_columns(const DevBox &B, int x0, int y0, int
 // division, a multiply and a subtraction.  The trilinear weights (6 a droplet)
 // are formed while staging, not 3 per node, the divisions by the cell volume
 // take div_by, and the merge keeps its 8 list heads in registers.
-// 16.8 M droplets on 256^3: 8.00 -> 4.96 ms (FP64 pipe 24%, issue 43%: the
-// rest is the latency of the merge at 16 warps per SM); 1 M on 128^3: 0.71 ->
-// 0.49 ms, where the edge tiles' merges from global memory counted most.
-template <int TX, int TY, int TZ>
-__global__ void __launch_bounds__(kDepositThreads, 2)
-k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P) {
-    step_kernel_begin();
+// 16.8 M droplets on 256^3: 8.00 -> 4.15 ms; 1 M on 128^3: 0.71 -> 0.39 ms, where
+// the edge tiles' merges from global memory counted most.  The rest is the
+// latency of the merge: more warps help, fewer instructions do not.
+template <int TX, int TY, int TZ, int CAP>
+__global__ void __launch_bounds__(kDepositThreads, 3)
+k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P, int *overflow_list) {
+    step_kernel_begin<false>();
     static_assert(TX * TY * TZ == kDepositThreads, "one thread per node of the tile");
-    constexpr int COLS = (TX + 1) * (TY + 1), CSW = TZ + 2, CAP = kDepCap64;
+    constexpr int COLS = (TX + 1) * (TY + 1), CSW = TZ + 2;
     extern __shared__ __align__(16) unsigned char sm[];
-    double *s_v = (double *)sm;                    // [V64_N][CAP]
-    int *s_lid = (int *)(sm + V64_N * CAP * 8);    // [CAP]
-    int *s_cs = s_lid + CAP, *s_off = s_cs + COLS * CSW;
+    double *s_w = (double *)sm;                        // [V64_N][CAP]
+    int *s_lid = (int *)(sm + V64_N * 8 * CAP);        // [CAP]
+    int *s_t = s_lid + CAP;                            // [CAP]
+    int *s_cs = s_t + CAP, *s_off = s_cs + COLS * CSW;
     const Tile tl = tiles[blockIdx.x];
     const DevBox &B = boxes[tl.box];
     const DevGrid &g = B.g;
@@ -490,14 +498,12 @@ k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams 
         if (staged) {
             // two droplets per pass: their loads are in flight together
             const DevState &O = B.st[B.cur];
-            const DevPayload &Y = B.pay;
             bool fast = g.rdV != nullptr;
-            auto stage = [&](int k, int c, const double *w, int l, int key) {
+            auto stage = [&](int k, int c, int t, const double *v, const double *w, int l, int key) {
                 s_lid[k] = l;
+                s_t[k] = t;
 #pragma unroll
-                for (int q = 0; q < 11; ++q) s_v[q * CAP + k] = w[3 + q];
-#pragma unroll
-                for (int q = 0; q < 10; ++q) fast = fast && plain_num(w[3 + q]);
+                for (int q = 0; q < P64_MULT; ++q) fast = fast && plain_num(v[q]);
                 // the weights of the cell's lower (0) and upper (1) nodes
                 const int ci = x0 - 1 + c / (TY + 1), cj = y0 - 1 + c % (TY + 1);
                 const int ck = key - (g.nnz + 1) * ((cj - 1) + (g.nny + 1) * (ci - 1));
@@ -508,9 +514,9 @@ k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams 
                     const double ay = fabs(w[1] - g.dy * (double)(cj + m + g.joff - 1));
                     const double az = fabs(w[2] - g.zz[ck + m]);
                     const bool f = g.rdV != nullptr;
-                    s_v[(V64_WX + m) * CAP + k] = 1.0 - (f ? div_by(ax, g.dx, g.rdx) : ax / g.dx);
-                    s_v[(V64_WY + m) * CAP + k] = 1.0 - (f ? div_by(ay, g.dy, g.rdy) : ay / g.dy);
-                    s_v[(V64_WZ + m) * CAP + k] = 1.0 - (f ? div_by(az, dz, g.rdzu[ck + 1]) : az / dz);
+                    s_w[(V64_WX + m) * CAP + k] = 1.0 - (f ? div_by(ax, g.dx, g.rdx) : ax / g.dx);
+                    s_w[(V64_WY + m) * CAP + k] = 1.0 - (f ? div_by(ay, g.dy, g.rdy) : ay / g.dy);
+                    s_w[(V64_WZ + m) * CAP + k] = 1.0 - (f ? div_by(az, dz, g.rdzu[ck + 1]) : az / dz);
                 }
             };
             for (int k0 = threadIdx.x; k0 < total; k0 += 2 * blockDim.x) {
@@ -521,17 +527,14 @@ k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams 
                 while (c1 + 1 < COLS && s_off[c1 + 1] <= k1) ++c1;
                 const int t0 = B.perm[s_cs[c0 * CSW] + (k0 - s_off[c0])];
                 const int t1 = two ? B.perm[s_cs[c1 * CSW] + (k1 - s_off[c1])] : t0;
-                const double *src[14] = {O.x[0], O.x[1], O.x[2], Y.D[0], Y.D[1], Y.D[2], Y.V[0],
-                                         Y.V[1], Y.V[2], Y.T0, Y.H0, Y.E1, Y.E2, Y.mult};
-                double w0[14], w1[14];
-#pragma unroll
-                for (int q = 0; q < 14; ++q) {
-                    w0[q] = src[q][t0];
-                    w1[q] = src[q][t1];
-                }
-                const int l0 = O.lid[t0], l1 = O.lid[t1], e0 = B.key[t0], e1 = B.key[t1];
-                stage(k0, c0, w0, l0, e0);
-                if (two) stage(k1, c1, w1, l1, e1);
+                double v0[P64_N], v1[P64_N];
+                int l0, l1, e0, e1;
+                load_payload64(B.pay, t0, v0, l0, e0);
+                load_payload64(B.pay, t1, v1, l1, e1);
+                const double w0[3] = {O.x[0][t0], O.x[1][t0], O.x[2][t0]};
+                const double w1[3] = {O.x[0][t1], O.x[1][t1], O.x[2][t1]};
+                stage(k0, c0, t0, v0, w0, l0, e0);
+                if (two) stage(k1, c1, t1, v1, w1, l1, e1);
             }
             fast = __syncthreads_and(fast) != 0;
             if (valid) {
@@ -551,14 +554,42 @@ k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams 
                         run[ij << 1 | k] = in ? (base + cs[0]) | (base + cs[1]) << 16 : 0;
                     }
                 }
-                if (fast) merge_staged64<true>(P, s_lid, s_v, run, dV, rdV, out);
-                else merge_staged64<false>(P, s_lid, s_v, run, dV, rdV, out);
+                if (fast) merge_staged64<true, CAP>(B, P, s_lid, s_t, s_w, run, dV, rdV, out);
+                else merge_staged64<false, CAP>(B, P, s_lid, s_t, s_w, run, dV, rdV, out);
             }
         }
+    }
+    if (!staged && overflow_list != nullptr) {
+        // above the stage capacity: k_deposit64_overflow, which has the
+        // registers of the global path
+        if (threadIdx.x == 0) overflow_list[1 + atomicAdd(overflow_list, 1)] = blockIdx.x;
+        return;
     }
     if (!valid) return;
     if (!staged) node_global64(B, P, ix, iy, iz, images, out);
     store_node(B, ix, iy, iz, out);
+}
+
+// FP64 tiles listed by k_deposit64: each node's own image merged from global
+// memory; grid-stride over the list
+template <int TX, int TY, int TZ>
+__global__ void __launch_bounds__(kDepositThreads, 2)
+k_deposit64_overflow(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P, const int *overflow_list) {
+    step_kernel_begin();
+    const int n = overflow_list[0];
+    for (int e = blockIdx.x; e < n; e += gridDim.x) {
+        const Tile tl = tiles[overflow_list[1 + e]];
+        const DevBox &B = boxes[tl.box];
+        const DevGrid &g = B.g;
+        const int ntz = (g.nz2 + TZ - 1) / TZ, nty = (g.dny + TY - 1) / TY;
+        const int tzi = tl.start % ntz, tyi = (tl.start / ntz) % nty, txi = tl.start / (ntz * nty);
+        const int lz = threadIdx.x % TZ, ly = (threadIdx.x / TZ) % TY, lx = threadIdx.x / (TZ * TY);
+        const int ix = 1 + txi * TX + lx, iy = 1 + tyi * TY + ly, iz = tzi * TZ + lz;
+        if (ix > g.dnx || iy > g.dny || iz > g.nnz + 1) continue;
+        double out[6];
+        image_global64(B, P, ix, iy, iz, out);
+        store_node(B, ix, iy, iz, out);
+    }
 }
 
 // Mixed tiles (z fastest), the same shapes.

@@ -115,9 +115,36 @@ struct DevState {
 
 // Deposition payload of one droplet (written by the update kernel in the
 // output order, read by the deposition kernel through the cell lists).
-struct DevPayload {
-    double *D[3], *V[3], *T0, *H0, *E1, *E2, *mult;
+// FP64: the reference's factors D and V of the momentum terms, T0, H0, E1, E2
+// and mult, with the droplet's lid and cell key, together in three 32-byte
+// words (see the mixed payload for why).  16.8 M droplets: deposition 4.96 ->
+// 4.69 ms with the words staged, 4.15 with them read in place.
+enum { P64_D = 0, P64_T0 = 3, P64_V = 4, P64_H0 = 7, P64_E1, P64_E2, P64_MULT, P64_N };
+constexpr int kPay64Words = 3;
+struct alignas(32) Quad64 {
+    double a, b, c, d;
 };
+struct DevPayload {
+    Quad64 *p;   // [cap][kPay64Words]; the last value: lid | key << 32
+};
+__device__ __forceinline__ Quad64 load_quad(const Quad64 *p) {
+    Quad64 v;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void store_quad(Quad64 *p, double a, double b, double c, double d) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+__device__ __forceinline__ void load_payload64(const DevPayload &y, int t, double v[P64_N], int &lid, int &key) {
+    const Quad64 *p = y.p + (long long)kPay64Words * t;
+    const Quad64 a = load_quad(p), b = load_quad(p + 1), c = load_quad(p + 2);
+    v[0] = a.a; v[1] = a.b; v[2] = a.c; v[3] = a.d;
+    v[4] = b.a; v[5] = b.b; v[6] = b.c; v[7] = b.d;
+    v[8] = c.a; v[9] = c.b; v[10] = c.c;
+    const long long w = __double_as_longlong(c.d);
+    lid = (int)w;
+    key = (int)(w >> 32);
+}
 
 // Mixed-precision payload, FP32: cell-relative position fractions
 // fx = (x - x_node)/dx etc. (the trilinear weights are fx and 1 - fx), the

@@ -391,7 +391,7 @@ k_update_rk3_64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevPar
         } else {
             key = cell_key(B.g, x[0], x[1], x[2]);
             if (in.write_payload)
-                write_payload(B, p, t, x, v, vold, radius, rold, Tp, Tpold, Tf, m_s, multi, dt);
+                write_payload(B, p, t, x, v, vold, radius, rold, Tp, Tpold, Tf, m_s, multi, dt, S.lid[s], key);
         }
         B.key[t] = key;
         atomicAdd(&B.cell_cnt[key], 1);   // the sort's histogram
@@ -412,7 +412,8 @@ __global__ void k_payload64(DevBox *boxes, const Tile *tiles, const __grid_const
     const int s = B.perm[t];
     double x[3], v[3], vold[3];
     for (int a = 0; a < 3; ++a) { x[a] = S.x[a][s]; v[a] = S.v[a][s]; vold[a] = S.vold[a][s]; }
-    write_payload(B, p, s, x, v, vold, S.r[s], S.rold[s], S.Tp[s], S.Tpold[s], S.Tf[s], S.m_s[s], S.mult[s], dt);
+    write_payload(B, p, s, x, v, vold, S.r[s], S.rold[s], S.Tp[s], S.Tpold[s], S.Tf[s], S.m_s[s], S.mult[s], dt,
+                  S.lid[s], B.key[s]);
 }
 
 // ---------------------------------------------------------------------------
@@ -448,34 +449,47 @@ void launch_payload64(DevBox *boxes, const Tile *tiles, int ntiles, const DevPar
     k_payload64<<<ntiles, kUpdateThreads, 0, st>>>(boxes, tiles, P, dt);
 }
 
-template <int V>
-static void dep64(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P, cudaStream_t st) {
-    constexpr int TX = kDepShape[V][0], TY = kDepShape[V][1], TZ = kDepShape[V][2];
-    launch_step_kernel(k_deposit64<TX, TY, TZ>, ntiles, kDepositThreads, dep_smem_bytes(false, TX, TY, TZ), st, boxes, tiles, P);
+template <int V, int C>
+static void dep64(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P, cudaStream_t st,
+                  int *overflow_list) {
+    constexpr int TX = kDepShape[V][0], TY = kDepShape[V][1], TZ = kDepShape[V][2], CAP = kDepCap64[C];
+    launch_step_kernel(k_deposit64<TX, TY, TZ, CAP>, ntiles, kDepositThreads,
+                       dep_smem_bytes(false, TX, TY, TZ) + CAP * kStage64, st, boxes, tiles, P, overflow_list);
+    if (overflow_list)
+        launch_step_kernel(k_deposit64_overflow<TX, TY, TZ>, ntiles < kOverflowBlocks ? ntiles : kOverflowBlocks,
+                           kDepositThreads, 0, st, boxes, tiles, P, overflow_list);
+}
+
+template <int V, int C>
+static void dep64_attr() {
+    constexpr int TX = kDepShape[V][0], TY = kDepShape[V][1], TZ = kDepShape[V][2], CAP = kDepCap64[C];
+    cudaFuncSetAttribute(k_deposit64<TX, TY, TZ, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         dep_smem_bytes(false, TX, TY, TZ) + CAP * kStage64);
 }
 
 template <int V>
-static void dep64_attr() {
-    constexpr int TX = kDepShape[V][0], TY = kDepShape[V][1], TZ = kDepShape[V][2];
-    cudaFuncSetAttribute(k_deposit64<TX, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         dep_smem_bytes(false, TX, TY, TZ));
+static void dep64_attrs() {
+    dep64_attr<V, 0>();
+    dep64_attr<V, 1>();
+    dep64_attr<V, 2>();
 }
 
 void prepare_kernels64() {
     if (!first_on_device(ONCE_DEP64)) return;
-    dep64_attr<0>();
-    dep64_attr<1>();
-    dep64_attr<2>();
+    dep64_attrs<0>();
+    dep64_attrs<1>();
+    dep64_attrs<2>();
 }
 
 void launch_deposit64(int variant, DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P,
-                      cudaStream_t st, int nbox) {
+                      cudaStream_t st, int nbox, int cap, int *overflow_list) {
     if (ntiles <= 0) return;
     prepare_kernels64();
-    if (variant == 1) dep64<1>(boxes, tiles, ntiles, P, st);
-    else if (variant == 2) dep64<2>(boxes, tiles, ntiles, P, st);
-    else dep64<0>(boxes, tiles, ntiles, P, st);
-    if (nbox > 0) launch_step_kernel(k_fold, dim3(kFoldBlocks, nbox), 256, 0, st, boxes, nullptr);
+    auto go = [&](auto dep) { dep(boxes, tiles, ntiles, P, st, overflow_list); };
+    if (variant == 1) go(cap == 0 ? dep64<1, 0> : cap == 1 ? dep64<1, 1> : dep64<1, 2>);
+    else if (variant == 2) go(cap == 0 ? dep64<2, 0> : cap == 1 ? dep64<2, 1> : dep64<2, 2>);
+    else go(cap == 0 ? dep64<0, 0> : cap == 1 ? dep64<0, 1> : dep64<0, 2>);
+    if (nbox > 0) launch_step_kernel(k_fold, dim3(kFoldBlocks, nbox), 256, 0, st, boxes, overflow_list);
 }
 
 }  // namespace ntlp

@@ -52,7 +52,7 @@ constexpr long long kOffSmall = kOffGrid + align256(4 * (kMaxNz + 3) * 8);      
 constexpr long long kOffFlux = kOffSmall + 256;                                     // pflux, flux_fx (unused)
 constexpr long long kOffInts = kOffFlux + align256((kMaxNz + 1) * 8 + 2 * (kMaxNz + 1) * kFluxLimbs * 8);
 constexpr long long kOffPay = kOffInts + align256(4 * kMaxN * 4);                    // lid, key, sorted, perm
-constexpr long long kOffCells = kOffPay + align256(11 * kMaxN * 8);
+constexpr long long kOffCells = kOffPay + align256(kPay64Words * kMaxN * (long long)sizeof(Quad64));
 constexpr long long kDropTiles = kMaxN / kUpdateThreads + 1;
 constexpr long long kCellTiles = (kMaxCells + 2) / kScanTile + 2;
 constexpr long long kNodeTiles = kMaxCells / 4 + 2;   // deposit tiles <= cells/4
@@ -182,13 +182,7 @@ extern "C" int ntlp_coupling_noalloc(const ntlp_grid *grid, const ntlp_params *p
         s.Tpold = (double *)d->Tp_old; s.Tf = (double *)d->Tf; s.m_s = (double *)d->m_s;
         s.mult = (long long *)d->mult; s.lid = lid;
     }
-    double *pay = (double *)(S + kOffPay);
-    for (int a = 0; a < 3; ++a) {
-        B.pay.D[a] = pay + a * kMaxN;
-        B.pay.V[a] = pay + (3 + a) * kMaxN;
-    }
-    B.pay.T0 = pay + 6 * kMaxN; B.pay.H0 = pay + 7 * kMaxN; B.pay.E1 = pay + 8 * kMaxN;
-    B.pay.E2 = pay + 9 * kMaxN; B.pay.mult = pay + 10 * kMaxN;
+    B.pay.p = (Quad64 *)(S + kOffPay);
     B.cur = 0;
     B.cap = (int)n;
     B.n_alive = (int *)(S + kOffSmall);
@@ -246,7 +240,7 @@ extern "C" int ntlp_coupling_noalloc(const ntlp_grid *grid, const ntlp_params *p
     launch_sort(B_d, plan, st);
     launch_finish(B_d, 1, st);
     launch_payload64(B_d, drop_tiles, nd, dp, dt, st);
-    launch_deposit64(0, B_d, node_tiles, nn, dp, st, 0);
+    launch_deposit64(0, B_d, node_tiles, nn, dp, st, 0, deposit64_cap((double)n / (double)ncells), nullptr);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         fprintf(stderr, "ntlp_coupling_noalloc: %s\n", cudaGetErrorString(e));

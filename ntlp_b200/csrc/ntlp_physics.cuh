@@ -634,7 +634,7 @@ __device__ __forceinline__ int apply_bcs(const DevBox &B, const DevParams &p, do
 __device__ __forceinline__ void write_payload(const DevBox &B, const DevParams &p, int t, const double x[3],
                                               const double v[3], const double vold[3], double r, double rold,
                                               double Tp, double Tpold, double Tf, double m_s, long long mult,
-                                              double dt) {
+                                              double dt, int lid, int key) {
     const double pi2 = p.pi2;
     double vrhs[3];
     for (int a = 0; a < 3; ++a) vrhs[a] = (v[a] - vold[a]) / dt;
@@ -650,16 +650,17 @@ __device__ __forceinline__ void write_payload(const DevBox &B, const DevParams &
     double partmass = rhop * 2.0 / 3.0 * pi2 * cube(r);
     double taup_i = 18.0 * rhoa * p.nuf / rhop / ((2.0 * r) * (2.0 * r));
     double H0 = p.rhow / rhoa * pi2 * 2.0 * (r * r) * radrhs;
-    const DevPayload &P = B.pay;
+    double D[3], V[3];
     for (int a = 0; a < 3; ++a) {
-        P.D[a][t] = partmass / rhoa * (vrhs[a] - p.g[a]);
-        P.V[a][t] = H0 * v[a];
+        D[a] = partmass / rhoa * (vrhs[a] - p.g[a]);
+        V[a] = H0 * v[a];
     }
-    P.T0[t] = (Tprhs_s * 6.0 * p.rhow / rhop / p.CpaCpp / taup_i * (pi2 / 2.0) * r * p.nuf);
-    P.H0[t] = H0;
-    P.E1[t] = H0 * p.Cpv / p.Cpa * Tp;
-    P.E2[t] = H0 * p.Cpv / p.Cpa * Tf;
-    P.mult[t] = (double)mult;
+    const double T0 = (Tprhs_s * 6.0 * p.rhow / rhop / p.CpaCpp / taup_i * (pi2 / 2.0) * r * p.nuf);
+    Quad64 *w = B.pay.p + (long long)kPay64Words * t;
+    store_quad(w, D[0], D[1], D[2], T0);
+    store_quad(w + 1, V[0], V[1], V[2], H0);
+    store_quad(w + 2, H0 * p.Cpv / p.Cpa * Tp, H0 * p.Cpv / p.Cpa * Tf, (double)mult,
+               __longlong_as_double((long long)(unsigned)lid | (long long)key << 32));
 }
 
 
@@ -998,7 +999,7 @@ __device__ __forceinline__ int be_body(const DevBox &B, const DevParams &p, cons
                 write_payload_mixed(B, p, t, ipt, jpt, kpt, x, v, vold, radius, rold, Tp, Tpold, Tf, m_s, multi,
                                     in.inv_dt);
             else
-                write_payload(B, p, t, x, v, vold, radius, rold, Tp, Tpold, Tf, m_s, multi, dt);
+                write_payload(B, p, t, x, v, vold, radius, rold, Tp, Tpold, Tf, m_s, multi, dt, S.lid[s], key);
         }
     }
     B.key[t] = key;

@@ -48,3 +48,29 @@ def test_fp64_sources_bit_exact(grid_n, extent, tiny):
         for q in range(6):
             assert bitwise_equal(np.asarray(got[q]), want[q]), q
     s.close()
+
+
+# densities on both sides of each stage capacity of the FP64 tiles, and above all of them
+@pytest.mark.parametrize("n", [1300, 1450, 2600, 2900, 9000, 9500, 20000])
+@pytest.mark.gpu
+@pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")
+def test_fp64_stage_capacities(n):
+    import ntlp_b200
+    import pyoracle
+    params = gen.default_params(icase=0)
+    grid = gen.make_grid(9, 9, 12, 2.0, 2.0, 2.0)              # 1300 cells
+    fields = gen.make_fields(grid, 3, rms=0.3)
+    d = gen.make_droplets(grid, fields, params, n, 3)
+    ext = {k: gen.to_ext(grid, v) for k, v in fields.items()}
+    s = ntlp_b200.DropletStep(grid, params, capacity=n)
+    s.set_fields_ext(ext)
+    s.set_droplets(d)
+    s.particle_update_BE(1e-3, 2)
+    o = pyoracle.Oracle(grid, params, ext)
+    od = clone(d)
+    o.step_be(od, 1e-3, 2)
+    want, _ = o.coupling(od, 1e-3)
+    for _ in range(2):                                         # the overflow list is empty again
+        for q, got in enumerate(s.particle_coupling_update(1e-3)):
+            assert bitwise_equal(np.asarray(got), want[q]), q
+    s.close()
