@@ -1195,10 +1195,15 @@ int droplets_download(ntlp_ctx *c, int b, ntlp_droplets *d) {
     rc |= get(S.radrhs, d->radrhs);
     rc |= get(S.mult, d->mult);
     if (rc) return rc;
-    launch_gather_list(here, slot, n, c->stream);
+    // the records take the other state buffer, which holds nothing between steps:
+    // its first 16 arrays (of cap values each, in one piece)
+    const DevState &T = B.st[1 - B.cur];
+    launch_list_records(here, B.perm, slot, n, (Quad64 *)T.x[0], c->stream);
     if (d->lid) {
         const bool direct = on_device(c, d->lid, 4);
-        launch_gather_list_i32(S.lid, slot, direct ? d->lid : (int *)h.staging, n, c->stream);
+        int *out = direct ? d->lid : (int *)h.staging;
+        if (n == h.n_uploaded) k_iota<<<(n + 255) / 256, 256, 0, c->stream>>>(out, n);
+        else launch_gather_list_i32(S.lid, slot, out, n, c->stream);
         if (!direct) CK(cudaMemcpyAsync(d->lid, h.staging, (size_t)n * 4, cudaMemcpyDefault, c->stream));
     }
     CK(cudaStreamSynchronize(c->stream));

@@ -183,6 +183,10 @@ struct ListGather {
     int n;
 };
 void launch_gather_list(const ListGather &g, const int *slot, int n, cudaStream_t st);
+// the same through records of kRecordValues values at a time; rec: kRecordValues
+// * 8 bytes for each slot of the state
+constexpr int kRecordValues = 16;
+void launch_list_records(const ListGather &g, const int *perm, const int *slot, int n, Quad64 *rec, cudaStream_t st);
 void launch_gather_list_i32(const int *src, const int *slot, int *dst, int n, cudaStream_t st);
 
 // x-y column subdomains (ntlp_subdomain.cu)

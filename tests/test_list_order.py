@@ -70,3 +70,37 @@ def test_rank_within_a_cell(n):
     for q, got in enumerate(s.particle_coupling_update(1e-4)):
         assert np.array_equal(np.asarray(got).view(np.int64), want[q].view(np.int64)), q
     s.close()
+
+
+# device read-backs of few and of many arrays: direct gathers up to two values,
+# records of 4, 8, 12 and 16, and more than one record
+@pytest.mark.parametrize("keys", [("Tp",), ("Tp", "radius"), ("xp",), ("xp", "Tp"), ("xp", "vp", "rc"), ("xp", "vp", "uf"),
+                                  ("xp", "vp", "uf", "vp_old", "Tp", "Tf", "radius"),
+                                  ("xp", "vp", "uf", "vp_old", "Tp", "Tf", "radius", "qinf", "qstar", "mult", "lid")])
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.gpu
+@pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")
+def test_device_read_back_of_any_arrays(keys, precision):
+    import ntlp_b200
+    case = small_case(n=1500, grid_n=(12, 10, 16), params=gen.default_params(icase=1, precision=precision))
+    d = clone(case.droplets)
+    d["xp"][2][::5] = 0.1 * d["radius"][::5]               # some die at the floor
+    d["vp"][2][::5] = -5.0
+    s = ntlp_b200.DropletStep(case.grid, case.params, capacity=1700)
+    s.set_fields_ext(case.ext())
+    s.set_droplets(d)
+    for it in (2, 3):
+        s.particle_update_BE(case.dt, it)
+        dev = s.get_droplets_device(keys=keys)             # between steps: the next one must not notice
+        host = s.get_droplets()
+        for k in keys:
+            assert np.array_equal(dev[k].cpu().numpy(), host[k]), (it, k)
+    s.close()
+    t = ntlp_b200.DropletStep(case.grid, case.params, capacity=1700)
+    t.set_fields_ext(case.ext())
+    t.set_droplets(d)
+    for it in (2, 3):
+        t.particle_update_BE(case.dt, it)
+    for k, v in t.get_droplets().items():
+        assert np.array_equal(v, host[k]), k
+    t.close()
