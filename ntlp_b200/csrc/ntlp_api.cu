@@ -599,15 +599,38 @@ void phase_end(ntlp_ctx *c, int phase, cudaEvent_t a) {
     c->recs.push_back({phase, a, b});
 }
 
-// whether kernels of this context can write p as elements of `align` bytes:
-// memory of its own device, aligned (anything else goes through a copy)
-bool on_device(ntlp_ctx *c, const void *p, size_t align) {
+// the allocation that holds a device pointer, from the driver
+typedef CUresult (*AddressRangeFn)(CUdeviceptr *, size_t *, CUdeviceptr);
+AddressRangeFn address_range_fn() {
+    static AddressRangeFn fn = []() -> AddressRangeFn {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult res;
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &p, 3020, cudaEnableDefault, &res) !=
+                cudaSuccess ||
+            res != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return (AddressRangeFn)p;
+    }();
+    return fn;
+}
+
+// Whether kernels of this context can read or write `count` elements of `size`
+// bytes at p: memory of its own device, aligned, within one allocation.
+// Anything else goes through a copy, which refuses what it cannot reach.
+bool on_device(ntlp_ctx *c, const void *p, size_t count, size_t size) {
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return a.type == cudaMemoryTypeDevice && a.device == c->device && (uintptr_t)p % align == 0;
+    if (a.type != cudaMemoryTypeDevice || a.device != c->device || (uintptr_t)p % size != 0) return false;
+    AddressRangeFn range = address_range_fn();
+    CUdeviceptr base = 0;
+    size_t bytes = 0;
+    if (!range || range(&base, &bytes, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS) return false;
+    return (CUdeviceptr)(uintptr_t)p - base + count * size <= bytes;
 }
 
 bool box_ok(ntlp_ctx *c, int b) { return c && b >= 0 && b < c->nbox; }
@@ -975,7 +998,7 @@ int fields_in(ntlp_ctx *c, int b, const double *const h[5], bool flow) {
     FieldSrc here{};
     bool any = false;
     for (int k = 0; k < 5; ++k) {
-        if (on_device(c, h[k], 8)) {
+        if (on_device(c, h[k], n, 8)) {
             here.p[k] = h[k];
             any = true;
             continue;
@@ -1170,7 +1193,7 @@ int droplets_download(ntlp_ctx *c, int b, ntlp_droplets *d) {
     auto get = [&](const void *src, void *dst) -> int {
         if (!dst || !src) return NTLP_OK;
         ListGather one{};
-        const bool direct = on_device(c, dst, 8);
+        const bool direct = on_device(c, dst, (size_t)n, 8);
         ListGather &g = direct ? here : one;
         g.src[g.n] = (const double *)src;
         g.dst[g.n++] = direct ? (double *)dst : h.staging;
@@ -1200,7 +1223,7 @@ int droplets_download(ntlp_ctx *c, int b, ntlp_droplets *d) {
     const DevState &T = B.st[1 - B.cur];
     launch_list_records(here, B.perm, slot, n, (Quad64 *)T.x[0], c->stream);
     if (d->lid) {
-        const bool direct = on_device(c, d->lid, 4);
+        const bool direct = on_device(c, d->lid, (size_t)n, 4);
         int *out = direct ? d->lid : (int *)h.staging;
         if (n == h.n_uploaded) k_iota<<<(n + 255) / 256, 256, 0, c->stream>>>(out, n);
         else launch_gather_list_i32(S.lid, slot, out, n, c->stream);
@@ -1362,7 +1385,7 @@ int sources_out(ntlp_ctx *c, int b, int32_t layout, double *const host[6]) {
         if (!host[q]) continue;
         any = true;
         const double *src = B.src[q];
-        if (layout == NTLP_LAYOUT_COLUMN && on_device(c, host[q], 8)) {
+        if (layout == NTLP_LAYOUT_COLUMN && on_device(c, host[q], (size_t)nn, 8)) {
             from.p[q] = B.src[q];
             here.p[q] = host[q];
             direct = true;
