@@ -366,37 +366,39 @@ __device__ __forceinline__ void store_node(const DevBox &B, int ix, int iy, int 
 
 // Periodic boxes: the fold of particle_coupling_exchange on the nodes
 // with ix <= 2 or iy <= 2, from their own image (in the sources) and the
-// image nodes, in node_fold's order; grid.y = box
+// image nodes, in node_fold's order; grid (blocks, boxes, quantities)
 __global__ void k_fold(DevBox *boxes, int *overflow_list) {
     step_kernel_begin();
     // the tiles listed for k_deposit_overflow32 are done: an empty list for the next deposition
-    if (overflow_list != nullptr && blockIdx.x + blockIdx.y + threadIdx.x == 0) overflow_list[0] = 0;
+    if (overflow_list != nullptr && blockIdx.x + blockIdx.y + blockIdx.z + threadIdx.x == 0)
+        overflow_list[0] = 0;
     const DevBox &B = boxes[blockIdx.y];
     const DevGrid &g = B.g;
     if (!g.periodic || B.img == nullptr || B.cellsum != nullptr) return;
     const int ya = g.nny < 2 ? g.nny : 2, xb = g.nnx < 2 ? g.nnx : 2;
-    const long long na = (long long)ya * g.nnx * g.nz2;                       // iy <= 2, every ix
-    const long long nb = g.nny > 2 ? (long long)xb * (g.nny - 2) * g.nz2 : 0;  // ix <= 2, iy >= 3
-    const long long per = img_count(g);
-    // a thread per (quantity, node): one node's six values in turn made a chain
-    // of loads, 14 us even in a 32^3 box
-    for (long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x; at < 6 * (na + nb);
-         at += (long long)gridDim.x * blockDim.x) {
-        const int q = (int)(at / (na + nb));
-        const long long idx = at - q * (na + nb);
+    // A thread per (quantity, node): one node's six values in turn made a chain
+    // of loads, 14 us even in a 32^3 box; grid.z is the quantity.  The padded grid has
+    // more points than there are border nodes, and fewer than 2^31: 32-bit divisions.
+    // Bound by the latency of its loads: kFoldBlocks has the measurements.
+    const unsigned nz2 = (unsigned)g.nz2, rows = (unsigned)(g.nny - 2);
+    const unsigned na = (unsigned)ya * g.nnx * nz2;                 // iy <= 2, every ix
+    const unsigned nb = g.nny > 2 ? (unsigned)xb * rows * nz2 : 0;  // ix <= 2, iy >= 3
+    const int q = blockIdx.z;
+    const double *I = B.img + q * img_count(g);
+    for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < na + nb; idx += gridDim.x * blockDim.x) {
         int ix, iy, iz;
         if (idx < na) {
-            iz = (int)(idx % g.nz2);
-            iy = 1 + (int)((idx / g.nz2) % ya);
-            ix = 1 + (int)(idx / ((long long)g.nz2 * ya));
+            const unsigned c = idx / nz2;
+            iz = (int)(idx - c * nz2);
+            iy = 1 + (int)(c % (unsigned)ya);
+            ix = 1 + (int)(c / (unsigned)ya);
         } else {
-            const long long r = idx - na;
-            iz = (int)(r % g.nz2);
-            iy = 3 + (int)((r / g.nz2) % (g.nny - 2));
-            ix = 1 + (int)(r / ((long long)g.nz2 * (g.nny - 2)));
+            const unsigned r = idx - na, c = r / nz2;
+            iz = (int)(r - c * nz2);
+            iy = 3 + (int)(c % rows);
+            ix = 1 + (int)(c / rows);
         }
         const long long node = (long long)iz + (long long)g.nz2 * ((long long)(iy - 1) + (long long)g.sny * (ix - 1));
-        const double *I = B.img + q * per;
         double out = B.src[q][node];
         if (ix <= 2) out = out + I[img_index(g, ix + g.nnx, iy, iz)];
         if (iy <= 2) {

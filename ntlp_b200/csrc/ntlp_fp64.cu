@@ -489,7 +489,7 @@ void launch_deposit64(int variant, DevBox *boxes, const Tile *tiles, int ntiles,
     if (variant == 1) go(cap == 0 ? dep64<1, 0> : cap == 1 ? dep64<1, 1> : dep64<1, 2>);
     else if (variant == 2) go(cap == 0 ? dep64<2, 0> : cap == 1 ? dep64<2, 1> : dep64<2, 2>);
     else go(cap == 0 ? dep64<0, 0> : cap == 1 ? dep64<0, 1> : dep64<0, 2>);
-    if (nbox > 0) launch_step_kernel(k_fold, dim3(kFoldBlocks, nbox), 256, 0, st, boxes, overflow_list);
+    if (nbox > 0) launch_step_kernel(k_fold, dim3(kFoldBlocks, nbox, 6), 256, 0, st, boxes, overflow_list);
 }
 
 }  // namespace ntlp

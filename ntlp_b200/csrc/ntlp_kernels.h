@@ -136,7 +136,12 @@ void launch_deposit_mixed(int variant, DevBox *boxes, const Tile *tiles, int nti
                           cudaStream_t st, int nbox, bool dense, int *overflow_list);
 constexpr int kDenseRatio = 16;     // mixed boxes with capacity >= 16 x cells use per-cell sums
 constexpr int kDenseBlocks = 1184;  // grid.x of the cell-sum kernels
-constexpr int kFoldBlocks = 148;    // grid.x of the periodic fold
+// grid.x of the periodic fold (x boxes x 6 quantities).  Deposition with one grid of 148
+// blocks over (quantity, node), with 50 and with 100 blocks a quantity: 1 M droplets on
+// 128^3 0.213 / 0.203 / 0.201 ms (FP64 0.391 / 0.380 / 0.378), 10,000 on 32^3 0.0197 /
+// 0.0181 / 0.0183; 16.8 M on 256^3 1.822 -> 1.774.  Twice as many gave 0.002 to
+// 0.004 ms on the large boxes and took as much back on the small.
+constexpr int kFoldBlocks = 100;
 // kernel attributes (dynamic shared memory of the deposition), set once per
 // device, on the device that is current; call outside stream capture
 void prepare_kernels64();

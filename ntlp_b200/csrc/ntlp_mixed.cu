@@ -681,7 +681,7 @@ void launch_deposit_mixed(int variant, DevBox *boxes, const Tile *tiles, int nti
     if (variant == 1) depm<1>(boxes, tiles, ntiles, P, st, overflow_list, dense);
     else if (variant == 2) depm<2>(boxes, tiles, ntiles, P, st, overflow_list, dense);
     else depm<0>(boxes, tiles, ntiles, P, st, overflow_list, dense);
-    launch_step_kernel(k_fold, dim3(kFoldBlocks, nbox), 256, 0, st, boxes, overflow_list);
+    launch_step_kernel(k_fold, dim3(kFoldBlocks, nbox, 6), 256, 0, st, boxes, overflow_list);
     if (dense) {
         launch_step_kernel(k_cellsums32, dim3(kDenseBlocks, nbox), 256, 0, st, boxes, P);
         launch_step_kernel(k_nodes_dense32, dim3(kDenseBlocks, nbox), 256, 0, st, boxes);

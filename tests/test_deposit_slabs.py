@@ -33,3 +33,13 @@ def test_slabs_match_cell_sums(grid_n, n):
         s.close()
     for q in range(6):
         assert bitwise_equal(out[0][q], out[1][q]), q
+
+
+@pytest.mark.parametrize("grid_n", [(2, 7, 5), (7, 2, 5), (2, 3, 4), (3, 2, 4), (90, 3, 60), (3, 90, 60)])
+@pytest.mark.gpu
+@pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")
+def test_fold_of_thin_boxes(grid_n):
+    """Boxes whose border nodes are all or most of them, and more than one round of
+    the fold's blocks: the images folded by a kernel of its own against the folded
+    cell sums.  The sources are the same bits."""
+    test_slabs_match_cell_sums(grid_n, 3_000)
