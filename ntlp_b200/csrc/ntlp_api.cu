@@ -35,6 +35,7 @@
 #include "ntlp_dev.cuh"
 #include "ntlp_kernels.h"
 #include "ntlp_math.h"
+#include "ntlp_overflow.h"
 
 using namespace ntlp;
 
@@ -101,7 +102,8 @@ struct ntlp_ctx {
     int n_dep_tiles[kDepVariants] = {};
     long long *tile_sums_d = nullptr;
     int *box_first_tile_d = nullptr;
-    int *overflow_list_d = nullptr;   // mixed deposition: tiles left to the global-memory kernel
+    int *overflow_list_d = nullptr;   // tiles that the deposition left to its global-memory kernel
+    OverflowState overflow;
     void *small_arena = nullptr;
     SortPlan plan{};
     int dep_variant = 0, nt_variant = 0;
@@ -1246,6 +1248,33 @@ bool staged_interp(const ntlp_ctx *c) {
     return c->blk_on && c->blk_kb > 0 && (!c->blk_auto || c->blk_pays);
 }
 
+// empties the overflow list if a deposition was launched in part; outside
+// stream capture, before the work that deposits
+int overflow_ready(ntlp_ctx *c) {
+    if (c->overflow.ready([&] { return (int)cudaMemsetAsync(c->overflow_list_d, 0, sizeof(int), c->stream); }))
+        return fail(c, NTLP_ERR_CUDA, "clearing the overflow list failed: %s",
+                    cudaGetErrorString(cudaGetLastError()));
+    return NTLP_OK;
+}
+
+// launch the kernels of one deposition (no synchronisation; graph-capturable)
+int launch_deposit(ntlp_ctx *c) {
+    cudaEvent_t e0 = phase_begin(c);
+    const int v = c->dep_variant;
+    c->overflow.begin();
+    if (c->params.precision == NTLP_PREC_MIXED)
+        launch_deposit_mixed(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
+                             c->any_dense, c->overflow_list_d);
+    else
+        launch_deposit64(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
+                         c->dep64_cap, c->overflow_list_d);
+    phase_end(c, PH_DEPOSIT, e0);
+    c->launches += deposit_launches(c);
+    CK(cudaGetLastError());
+    c->overflow.end();
+    return NTLP_OK;
+}
+
 // launch the kernels of one step (no synchronisation; graph-capturable)
 int launch_step(ntlp_ctx *c, int kind, int istage, double dt, int32_t it, bool with_deposit) {
     const int nt = kNtValues[c->nt_variant];
@@ -1280,18 +1309,7 @@ int launch_step(ntlp_ctx *c, int kind, int istage, double dt, int32_t it, bool w
     launch_finish(c->box_d, c->nbox, c->stream);
     phase_end(c, PH_SORT, e0);
     c->launches += 1 + kSortLaunches + 1;
-    if (with_deposit) {
-        e0 = phase_begin(c);
-        const int v = c->dep_variant;
-        if (c->params.precision == NTLP_PREC_MIXED)
-            launch_deposit_mixed(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
-                                 c->any_dense, c->overflow_list_d);
-        else
-            launch_deposit64(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
-                             c->dep64_cap, c->overflow_list_d);
-        phase_end(c, PH_DEPOSIT, e0);
-        c->launches += deposit_launches(c);
-    }
+    if (with_deposit) return launch_deposit(c);
     CK(cudaGetLastError());
     return NTLP_OK;
 }
@@ -1458,7 +1476,7 @@ int stats_run(ntlp_ctx *c, int b, bool radius_hist) {
 // the deposition of particle_coupling_update on the context's stream
 int launch_coupling(ntlp_ctx *c, double dt) {
     int rc = wait_download(c);
-    if (rc) return rc;
+    if (rc || (rc = overflow_ready(c))) return rc;
     if (!c->payload_valid || c->last_dt != dt) {
         cudaEvent_t ep = phase_begin(c);
         if (c->params.precision == NTLP_PREC_MIXED)
@@ -1470,18 +1488,7 @@ int launch_coupling(ntlp_ctx *c, double dt) {
         c->payload_valid = true;
         c->last_dt = dt;
     }
-    cudaEvent_t e0 = phase_begin(c);
-    const int v = c->dep_variant;
-    if (c->params.precision == NTLP_PREC_MIXED)
-        launch_deposit_mixed(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
-                             c->any_dense, c->overflow_list_d);
-    else
-        launch_deposit64(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
-                             c->dep64_cap, c->overflow_list_d);
-    phase_end(c, PH_DEPOSIT, e0);
-    c->launches += deposit_launches(c);
-    CK(cudaGetLastError());
-    return NTLP_OK;
+    return launch_deposit(c);
 }
 
 // another block height for the staged interpolation: the boxes' tensor
@@ -1832,11 +1839,12 @@ static int build_graph(ntlp_ctx *c, double dt, int32_t it, int32_t nsteps) {
         cudaGraphExecDestroy(c->gexec);
         c->gexec = nullptr;
     }
+    int lrc = overflow_ready(c);   // not in the capture: an eager deposition may come before its launch
+    if (lrc) return lrc;
     const bool prof = c->prof;
     c->prof = false;   // no events inside the capture
     const int64_t launches = c->launches;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    int lrc = NTLP_OK;
     for (int s = 0; s < nsteps && !lrc; ++s) lrc = launch_step(c, 1, 0, dt, it, true);
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
@@ -1878,9 +1886,11 @@ int ntlp_advance_graph(ntlp_ctx *c, double dt, int32_t it, int32_t nsteps) {
     int rc = check_ready(c, dt);
     if (rc) return rc;
     if ((rc = consume_upload(c)) || (rc = wait_download(c))) return rc;
-    if ((rc = build_graph(c, dt, it, nsteps))) return rc;
+    if ((rc = build_graph(c, dt, it, nsteps)) || (rc = overflow_ready(c))) return rc;
     cudaEvent_t e0 = phase_begin(c);
+    c->overflow.begin();
     CK(cudaGraphLaunch(c->gexec, c->stream));
+    c->overflow.end();
     phase_end(c, PH_OTHER, e0);
     c->launches += c->g_launches;
     mirror_flip(c, nsteps);
@@ -1927,7 +1937,7 @@ int ntlp_autotune(ntlp_ctx *c, double dt, int32_t it, int32_t steps, int32_t cho
     if (!c) return NTLP_ERR_ARG;
     int rc = check_ready(c, dt);
     if (rc) return rc;
-    if ((rc = consume_upload(c)) || (rc = wait_download(c))) return rc;
+    if ((rc = consume_upload(c)) || (rc = wait_download(c)) || (rc = overflow_ready(c))) return rc;
     if (steps < 1) steps = 1;
     if (it < 2) it = 2;
     cudaEvent_t a, b;

@@ -31,6 +31,7 @@
 
 #include "ntlp_dev.cuh"
 #include "ntlp_kernels.h"
+#include "ntlp_overflow.h"
 
 namespace ntlp {
 namespace {
@@ -369,7 +370,7 @@ __device__ __forceinline__ void store_node(const DevBox &B, int ix, int iy, int 
 // image nodes, in node_fold's order; grid (blocks, boxes, quantities)
 __global__ void k_fold(DevBox *boxes, int *overflow_list) {
     step_kernel_begin();
-    // the tiles listed for k_deposit_overflow32 are done: an empty list for the next deposition
+    // the tiles listed for the overflow kernel are done: an empty list for the next deposition
     if (overflow_list != nullptr && blockIdx.x + blockIdx.y + blockIdx.z + threadIdx.x == 0)
         overflow_list[0] = 0;
     const DevBox &B = boxes[blockIdx.y];
@@ -564,7 +565,8 @@ k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams 
     if (!staged && overflow_list != nullptr) {
         // above the stage capacity: k_deposit64_overflow, which has the
         // registers of the global path
-        if (threadIdx.x == 0) overflow_list[1 + atomicAdd(overflow_list, 1)] = blockIdx.x;
+        if (threadIdx.x == 0)
+            overflow_put(overflow_list, gridDim.x, blockIdx.x, [](int *n) { return atomicAdd(n, 1); });
         return;
     }
     if (!valid) return;
@@ -576,9 +578,10 @@ k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams 
 // memory; grid-stride over the list
 template <int TX, int TY, int TZ>
 __global__ void __launch_bounds__(kDepositThreads, 2)
-k_deposit64_overflow(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P, const int *overflow_list) {
+k_deposit64_overflow(DevBox *boxes, const Tile *tiles, int ntiles, const __grid_constant__ DevParams P,
+                     const int *overflow_list) {
     step_kernel_begin();
-    const int n = overflow_list[0];
+    const int n = overflow_count(overflow_list, ntiles);
     for (int e = blockIdx.x; e < n; e += gridDim.x) {
         const Tile tl = tiles[overflow_list[1 + e]];
         const DevBox &B = boxes[tl.box];
@@ -630,7 +633,8 @@ k_deposit_tiled(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevPar
     if (total > CAP) {
         // above the stage capacity: k_deposit_overflow32, which has the
         // registers of the global path
-        if (threadIdx.x == 0) overflow_list[1 + atomicAdd(overflow_list, 1)] = blockIdx.x;
+        if (threadIdx.x == 0)
+            overflow_put(overflow_list, gridDim.x, blockIdx.x, [](int *n) { return atomicAdd(n, 1); });
         return;
     }
     // two droplets per pass: their perm and payload loads are in flight
@@ -704,9 +708,10 @@ k_deposit_tiled(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevPar
 // global memory, stored like the tiled kernel's; grid-stride over the list
 template <int kDepTX, int kDepTY, int kDepTZ>
 __global__ void __launch_bounds__(kDepositThreads)
-k_deposit_overflow32(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P, const int *overflow_list) {
+k_deposit_overflow32(DevBox *boxes, const Tile *tiles, int ntiles, const __grid_constant__ DevParams P,
+                     const int *overflow_list) {
     step_kernel_begin();
-    const int n = overflow_list[0];
+    const int n = overflow_count(overflow_list, ntiles);
     for (int e = blockIdx.x; e < n; e += gridDim.x) {
         const Tile tl = tiles[overflow_list[1 + e]];
         const DevBox &B = boxes[tl.box];

@@ -457,7 +457,7 @@ static void dep64(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams 
                        dep_smem_bytes(false, TX, TY, TZ) + CAP * kStage64, st, boxes, tiles, P, overflow_list);
     if (overflow_list)
         launch_step_kernel(k_deposit64_overflow<TX, TY, TZ>, ntiles < kOverflowBlocks ? ntiles : kOverflowBlocks,
-                           kDepositThreads, 0, st, boxes, tiles, P, overflow_list);
+                           kDepositThreads, 0, st, boxes, tiles, ntiles, P, overflow_list);
 }
 
 template <int V, int C>

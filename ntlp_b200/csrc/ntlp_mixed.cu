@@ -657,7 +657,8 @@ static void depm(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &
     launch_step_kernel(k_deposit_tiled<TX, TY, TZ>, ntiles, kDepositThreads, dep_smem_bytes(true, TX, TY, TZ), st, boxes, tiles, P, overflow_list,
                                                                            dense ? 1 : 0);
     const int g = ntiles < kDenseBlocks ? ntiles : kDenseBlocks;
-    launch_step_kernel(k_deposit_overflow32<TX, TY, TZ>, g, kDepositThreads, 0, st, boxes, tiles, P, overflow_list);
+    launch_step_kernel(k_deposit_overflow32<TX, TY, TZ>, g, kDepositThreads, 0, st, boxes, tiles, ntiles, P,
+                       overflow_list);
 }
 
 template <int V>
