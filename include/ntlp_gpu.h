@@ -208,11 +208,12 @@ int ntlp_stream_priority(ntlp_ctx *ctx, int32_t priority);
  * height in cells (blocks are 4 x 4 x height cells; the context picks one
  * from its droplets per cell, ntlp_autotune tries half and twice that)
  * and switches staging on.  Until a call sets it, the context stages only
- * where that is the faster of the two: in boxes of a million droplets or
- * more with 0.75 to 40 of them per cell.
- * Returns the block height in cells (0: switched off) or an error
- * code (< 0).  The results do not depend on it.  No counterpart in the
- * reference.                                                              */
+ * where that is the faster of the two: with room for a million droplets or
+ * more, 0.75 to 40 of them per cell.  What a call sets holds for the rest of
+ * the context's life.
+ * Returns the block height in cells that steps now run with (0: the
+ * per-droplet kernel) or an error code (< 0).  The results do not depend on
+ * it.  No counterpart in the reference.                                    */
 int ntlp_interp_staging(ntlp_ctx *ctx, int32_t enable);
 
 /* ---- instrumentation (phase timers; measurement.f90's named phases) ----- */

@@ -233,9 +233,10 @@ class DropletStep:
         self._check(self.L.ntlp_use_stream(self.h, C.c_void_p(stream_handle or None)), "ntlp_use_stream")
 
     def interp_staging(self, enable: int = -1) -> int:
-        """Mixed 6th-order interpolation over staged cell blocks (1) or per
-        droplet from global memory (0); -1 queries.  Returns the block
-        height in cells (0: per droplet)."""
+        """Mixed 6th-order interpolation over staged cell blocks (1; 4, 8, 16
+        or 32: blocks of that height) or per droplet from global memory (0);
+        -1 queries.  Returns the block height in cells that steps now run
+        with (0: per droplet).  Until it is set, the context chooses."""
         r = int(self.L.ntlp_interp_staging(self.h, int(enable)))
         if r < 0:
             self._check(r, "ntlp_interp_staging")

@@ -1275,6 +1275,9 @@ int launch_deposit(ntlp_ctx *c) {
     return NTLP_OK;
 }
 
+// block height that steps interpolate over, 0 when they run per droplet
+int running_blk_kb(const ntlp_ctx *c) { return staged_interp(c) ? c->blk_kb : 0; }
+
 // launch the kernels of one step (no synchronisation; graph-capturable)
 int launch_step(ntlp_ctx *c, int kind, int istage, double dt, int32_t it, bool with_deposit) {
     const int nt = kNtValues[c->nt_variant];
@@ -1628,7 +1631,7 @@ int ntlp_interp_staging(ntlp_ctx *c, int32_t enable) {
     } else if (enable != -1) {
         return fail(c, NTLP_ERR_ARG, "staging switch %d", enable);
     }
-    return c->blk_on ? c->blk_kb : 0;
+    return running_blk_kb(c);
 }
 
 int ntlp_profile_enable(ntlp_ctx *c, int enable) {
@@ -2007,7 +2010,7 @@ int ntlp_autotune(ntlp_ctx *c, double dt, int32_t it, int32_t steps, int32_t cho
     if (choice) {
         choice[0] = best_dep;
         choice[1] = best_nt;
-        choice[2] = c->blk_on ? c->blk_kb : 0;
+        choice[2] = running_blk_kb(c);
     }
     if (ms)
         for (int k = 0; k < NTLP_TUNE_VARIANTS; ++k) ms[k] = local[k];

@@ -149,8 +149,8 @@ def test_autotune_changes_no_result(precision):
     r = a.autotune(dt, 2, steps=1)          # 5 to 7 variants x 2 steps
     assert 0 <= r["deposit_variant"] < 3 and 0 <= r["block_variant"] < 2
     assert all(m > 0 for m in r["ms"][:5])
-    staged = precision == abi.NTLP_PREC_MIXED
-    assert (r["interp_block_height"] in (4, 8, 16, 32)) == staged
+    # 0: per droplet, in FP64 and in a mixed context that runs faster so
+    assert r["interp_block_height"] in ((0, 4, 8, 16, 32) if precision == abi.NTLP_PREC_MIXED else (0,))
     assert r["interp_block_height"] == a.interp_staging(-1)
     nsteps = r["steps_advanced"]
     assert nsteps == 2 * sum(1 for m in r["ms"] if m > 0) and nsteps >= 10

@@ -123,21 +123,22 @@ def test_staged_interpolation_in_a_batch():
             assert bitwise_equal(np.asarray(sa[q]), np.asarray(sb[q])), q
 
 
-@pytest.mark.parametrize("edge,n,height", [
-    (20, 2_000, 16),            # small: per droplet unless asked for
-    (40, 1_000_000, 4),         # dense enough and large enough: staged
-    (24, 1_000_000, 4),         # 64 per cell: per droplet
+@pytest.mark.parametrize("edge,n,runs,height", [
+    (20, 2_000, 0, 16),         # small: per droplet unless asked for
+    (40, 1_000_000, 4, 4),      # dense enough and large enough: staged
+    (24, 1_000_000, 0, 4),      # 64 per cell: per droplet
 ])
-def test_default_choice_gives_the_same_bits(edge, n, height):
+def test_default_choice_gives_the_same_bits(edge, n, runs, height):
     import ntlp_b200
     params = dict(gen.default_params(ilin=0), precision=abi.NTLP_PREC_MIXED)
     case = small_case(params=params, n=n, grid_n=(edge, edge, edge))
     out = []
     for setting in (None, 1, 0):
         s = ntlp_b200.DropletStep(case.grid, params, capacity=n)
-        assert s.interp_staging(-1) == height
+        assert s.interp_staging(-1) == runs
         if setting is not None:
             assert s.interp_staging(setting) == (height if setting else 0)
+            assert s.interp_staging(-1) == (height if setting else 0)
         s.set_fields_ext(case.ext())
         s.set_droplets(case.droplets)
         s.particle_update_BE(case.dt, 1)
@@ -145,3 +146,20 @@ def test_default_choice_gives_the_same_bits(edge, n, height):
         s.close()
     for k in STATE_KEYS:
         assert bitwise_equal(out[0][k], out[1][k]) and bitwise_equal(out[0][k], out[2][k]), k
+
+
+@pytest.mark.parametrize("edge,capacity,runs", [
+    (110, 1_025_723, 0),        # just below 0.75 per cell (111^3 cells)
+    (110, 1_025_724, 16),       # just above
+    (40, 999_999, 0),           # just below a million
+    (40, 1_000_000, 4),
+    (30, 1_191_639, 4),         # just below 40 per cell (31^3 cells)
+    (30, 1_191_640, 0),         # 40
+])
+def test_default_choice_on_both_sides_of_each_bound(edge, capacity, runs):
+    """Which kernel a context runs until it is told."""
+    import ntlp_b200
+    params = dict(gen.default_params(ilin=0), precision=abi.NTLP_PREC_MIXED)
+    s = ntlp_b200.DropletStep(gen.make_grid(edge, edge, edge, 1.0, 1.0, 1.0), params, capacity=capacity)
+    assert s.interp_staging(-1) == runs
+    s.close()
