@@ -206,7 +206,7 @@ int ntlp_stream_priority(ntlp_ctx *ctx, int32_t priority);
  * kernel (stencil from global memory; the same results, bit for bit), 1
  * back to the staged one, -1 only queries; 4, 8, 16 or 32 sets the block
  * height in cells (blocks are 4 x 4 x height cells; the context picks one
- * from its droplets per cell, ntlp_autotune tries half and twice that)
+ * from its droplets per cell, ntlp_autotune tries others)
  * and switches staging on.  Until a call sets it, the context stages only
  * where that is the faster of the two: with room for a million droplets or
  * more, 0.75 to 40 of them per cell.  What a call sets holds for the rest of
@@ -279,9 +279,10 @@ int ntlp_step_time(ntlp_ctx *ctx, int32_t slot, double *ms);
  * fastest, and reports the per-variant milliseconds per step (ms[i] for
  * deposition shape i, ms[3+j] for block size j).  With the staged mixed
  * interpolation it then times half and twice the context's block height
- * (ms[5], ms[6]; 0 when not tried, outside 4..32) and keeps the fastest.
+ * (ms[5], ms[6]; 0 when not tried, outside 4..32), in a context that runs per
+ * droplet by its own choice that height and twice it, and keeps the fastest.
  * choice = {deposition shape, block size, interpolation block height (0:
- * none)}.  The state advances by steps + 1 steps per variant timed.  No
+ * per droplet)}.  The state advances by steps + 1 steps per variant timed.  No
  * variant changes a result.                                               */
 #define NTLP_TUNE_VARIANTS 7
 int ntlp_autotune(ntlp_ctx *ctx, double dt, int32_t it, int32_t steps, int32_t choice[3],

@@ -395,9 +395,9 @@ class DropletStep:
         return out
 
     def autotune(self, dt: float, it: int, steps: int = 2) -> dict:
-        """Time the deposition tile shapes, the droplet block sizes and (staged
-        mixed interpolation) half and twice the interpolation block height on
-        this context's boxes, and keep the fastest.  The state advances by
+        """Time the deposition tile shapes, the droplet block sizes and (mixed,
+        6th order) two heights of the staged interpolation's blocks on this
+        context's boxes, and keep the fastest.  The state advances by
         steps + 1 steps per variant timed: `steps_advanced` in the result."""
         choice = (C.c_int32 * 3)()
         ms = (C.c_double * abi.NTLP_TUNE_VARIANTS)()

@@ -1976,15 +1976,16 @@ int ntlp_autotune(ntlp_ctx *c, double dt, int32_t it, int32_t steps, int32_t cho
         if (!rc && local[kDepVariants + v] < local[kDepVariants + best_nt]) best_nt = v;
     }
     c->nt_variant = best_nt;
-    // the staged interpolation's block height: the context's choice, half of
-    // it and twice it (within 4..32 and the tile table)
+    // the staged interpolation's block height (within 4..32 and the tile
+    // table): half of what was timed above and twice it; a context that ran
+    // per droplet above times its own height and twice that
     if (!rc && c->blk_kb > 0 && c->blk_on) {
         const int kb0 = c->blk_kb;
-        const bool automatic = c->blk_auto;
+        const bool automatic = c->blk_auto, staged = staged_interp(c);
         c->blk_auto = false;
-        int best_kb = kb0;
+        int best_kb = 0;   // none is better than what ran above
         double best_ms = local[kDepVariants + best_nt];
-        const int cand[2] = {kb0 / 2, kb0 * 2};
+        const int cand[2] = {staged ? kb0 / 2 : kb0, kb0 * 2};
         for (int i = 0; i < 2 && !rc; ++i) {
             const int kb = cand[i];
             if (kb < 4 || kb > 32) continue;
@@ -1998,8 +1999,8 @@ int ntlp_autotune(ntlp_ctx *c, double dt, int32_t it, int32_t steps, int32_t cho
                 best_kb = kb;
             }
         }
-        if (!rc) rc = set_blk_kb(c, best_kb);
-        if (best_kb == kb0) c->blk_auto = automatic;
+        if (!rc) rc = set_blk_kb(c, best_kb ? best_kb : kb0);
+        if (!best_kb) c->blk_auto = automatic;
     }
     c->prof = prof;
     cudaEventDestroy(a);

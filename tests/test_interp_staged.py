@@ -163,3 +163,41 @@ def test_default_choice_on_both_sides_of_each_bound(edge, capacity, runs):
     s = ntlp_b200.DropletStep(gen.make_grid(edge, edge, edge, 1.0, 1.0, 1.0), params, capacity=capacity)
     assert s.interp_staging(-1) == runs
     s.close()
+
+
+@pytest.mark.parametrize("n,height,setting,timed", [
+    (9_000, 4, None, (True, True)),     # runs per droplet: 4 itself and 8
+    (9_000, 4, 1, (False, True)),       # staged at 4: 2 is no height, and 8
+    (9_000, 4, 0, (False, False)),      # switched off
+    (900, 16, None, (True, True)),      # runs per droplet: 16 and 32
+])
+def test_autotuner_times_the_heights_not_run_by_default(n, height, setting, timed):
+    """Which block heights the tuner times, and that the context then runs what
+    it reports: the same bits as a context that is not tuned."""
+    import ntlp_b200
+    params = dict(gen.default_params(ilin=0), precision=abi.NTLP_PREC_MIXED)
+    case = small_case(params=params, n=n, grid_n=(8, 8, 12))
+    out = []
+    for tuned in (True, False):
+        s = ntlp_b200.DropletStep(case.grid, params, capacity=n)
+        assert s.interp_staging(-1) == 0
+        if setting is not None:
+            assert s.interp_staging(setting) == (height if setting else 0)
+        s.set_fields_ext(case.ext())
+        s.set_droplets(case.droplets)
+        if tuned:
+            r = s.autotune(case.dt, 2, steps=1)
+            assert tuple(m > 0 for m in r["ms"][5:]) == timed
+            fastest = min(r["ms"][3:5])
+            better = [kb for kb, m in zip((height if setting is None else height // 2, 2 * height), r["ms"][5:])
+                      if 0 < m < fastest]
+            assert r["interp_block_height"] == s.interp_staging(-1)
+            assert r["interp_block_height"] in (better or [height if setting == 1 else 0])
+            steps = r["steps_advanced"]
+        else:
+            for it in range(2, 2 + steps):
+                s.particle_update_BE(case.dt, it)
+        out.append(s.get_droplets())
+        s.close()
+    for k in STATE_KEYS:
+        assert bitwise_equal(out[0][k], out[1][k]), k
