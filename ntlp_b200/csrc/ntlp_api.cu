@@ -901,7 +901,7 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
             {
                 size_t mx = 0;
                 for (int v = 0; v < kDepVariants; ++v) mx = std::max(mx, dpt[v].size());
-                k.take(&c->overflow_list_d, 1 + mx);
+                k.take(&c->overflow_list_d, 2 + mx);
             }
             k.take(&c->dp_d, 1);
             k.take(&c->box_d, (size_t)nbox);

@@ -130,8 +130,8 @@ void launch_payload_mixed(DevBox *boxes, const Tile *tiles, int ntiles, const De
                           cudaStream_t st);
 // dense: some box has per-cell sums (cellsum), deposited by the cell-sum
 // kernels instead of the tiles
-// overflow_list: [1 + tiles] ints of scratch (count, then tile indices), the
-// count 0 on entry and on return
+// overflow_list: [2 + tiles] ints of scratch (ntlp_overflow.h), the count 0 on
+// entry and on return
 void launch_deposit_mixed(int variant, DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P,
                           cudaStream_t st, int nbox, bool dense, int *overflow_list);
 constexpr int kDenseRatio = 16;     // mixed boxes with capacity >= 16 x cells use per-cell sums

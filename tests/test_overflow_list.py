@@ -16,7 +16,7 @@ using namespace ntlp;
 static int add(int *n) { return (*n)++; }
 int main() {
     const int ntiles = 5, guard = -77;
-    std::vector<int> mem(1 + ntiles + 64, guard);
+    std::vector<int> mem(2 + ntiles + 64, guard);
     int *list = mem.data();
     list[0] = 0;
     OverflowState s;
@@ -36,7 +36,7 @@ int main() {
         s.end();
         for (int t = 0; t < ntiles; ++t) bad += seen[t] != 1;
     };
-    auto guards = [&] { for (size_t k = 1 + ntiles; k < mem.size(); ++k) bad += mem[k] != guard; };
+    auto guards = [&] { for (size_t k = 2 + ntiles; k < mem.size(); ++k) bad += mem[k] != guard; };
     bad += s.ready(clear) != 0; deposit(3);
     for (int at = 0; at < 3; ++at) {
         bad += s.ready(clear) != 0; deposit(at); guards();
