@@ -36,6 +36,7 @@
 #include "ntlp_kernels.h"
 #include "ntlp_math.h"
 #include "ntlp_overflow.h"
+#include "ntlp_stage64.h"
 
 using namespace ntlp;
 
@@ -100,6 +101,9 @@ struct ntlp_ctx {
     int n_cell_tiles = 0;
     Tile *dep_tiles_d[kDepVariants] = {};
     int n_dep_tiles[kDepVariants] = {};
+    // FP64: the order of the boxes in that table, and its runs by stage capacity
+    std::vector<int> dep_order[kDepVariants];
+    std::vector<TileRun> dep_runs[kDepVariants];
     long long *tile_sums_d = nullptr;
     int *box_first_tile_d = nullptr;
     int *overflow_list_d = nullptr;   // tiles that the deposition left to its global-memory kernel
@@ -107,7 +111,6 @@ struct ntlp_ctx {
     void *small_arena = nullptr;
     SortPlan plan{};
     int dep_variant = 0, nt_variant = 0;
-    int dep64_cap = 0;                // FP64 deposition: stage capacity (deposit64_cap)
     long long *counters_h = nullptr;   // pinned [nbox][kNumCounters]
     int *err_h = nullptr;              // pinned [nbox] device error words
     // device-timed steps (ntlp_step_timed): an event pair per slot
@@ -136,6 +139,7 @@ struct ntlp_ctx {
     int g_nsteps = 0, g_dep = -1, g_nt = -1;
     bool g_blk = false;
     int g_kb = 0;
+    std::vector<TileRun> g_runs;
     bool tex_all = true;   // every box's FP32 fields have a texture (mixed)
     // staged cell-block interpolation (mixed, 6th order): block height and
     // tiles; blk_kb = 0 when the tensor maps could not be made
@@ -726,6 +730,33 @@ bool deposit_reciprocals(const DevGrid &g, const std::vector<double> &dzu, std::
     return all;
 }
 
+// FP64 deposition: the runs of the tile tables by stage capacity, each box's
+// from the droplets it was given, not from its room for them (1 M droplets on
+// 128^3 with room for 6 M: 0.376 ms, as without; 0.959 by the room).  Where that
+// changes the order of the boxes, the table is written anew; the stream is
+// waited for.
+int deposit64_plan(ntlp_ctx *c) {
+    for (int v = 0; v < kDepVariants; ++v) {
+        std::vector<int> cap(c->nbox), tiles(c->nbox), order;
+        for (int b = 0; b < c->nbox; ++b) {
+            const DevGrid &g = c->box[b].g;
+            tiles[b] = (int)deposit_tile_count(v, g.dnx, g.dny, g.nnz);
+            cap[b] = deposit64_cap(c->bh[b].n_uploaded, g.ncells, deposit_tile_cells(v));
+        }
+        deposit64_order(cap, tiles, order, c->dep_runs[v]);
+        if (order == c->dep_order[v]) continue;
+        std::vector<Tile> table;
+        for (int b : order)
+            for (int s = 0; s < tiles[b]; ++s) table.push_back(Tile{b, s});
+        c->dep_order[v].clear();   // unknown until it is written
+        CK(cudaMemcpyAsync(c->dep_tiles_d[v], table.data(), table.size() * sizeof(Tile), cudaMemcpyHostToDevice,
+                           c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        c->dep_order[v] = order;
+    }
+    return NTLP_OK;
+}
+
 // an x-y column subdomain of the periodic domain (set_bounds,
 // particles.f90:1766-1781): the grid spacing is the global domain's
 void subdomain_geometry(const ntlp_grid &grid, const ntlp_subdomain &sd, DevBox &B) {
@@ -863,12 +894,6 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
             if (!encode_f4_map(c->box[b], c->blk_kb)) c->blk_kb = 0;
         for (int b = 0; b < nbox; ++b) c->box[b].blk_kb = c->blk_kb;
     }
-    if (!mixed) {
-        double density = 0.0;   // of the fullest box
-        for (int b = 0; b < nbox; ++b)
-            density = std::max(density, (double)c->bh[b].cap / (double)c->box[b].g.ncells);
-        c->dep64_cap = deposit64_cap(density);
-    }
     // tiles: droplets (128 and 256 per tile), cells (scan tiles), deposition
     // (3 shapes), interpolation cell blocks
     std::vector<Tile> dt[kNtVariants], ct, dpt[kDepVariants], bt;
@@ -952,6 +977,12 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
         cudaMallocHost((void **)&c->err_h, sizeof(int) * nbox) != cudaSuccess)
         return bail(fail(c, NTLP_ERR_NOMEM, "pinned counter buffer refused"));
     if (push_boxes(c)) return bail(NTLP_ERR_CUDA);
+    if (!mixed) {
+        // no droplets yet: the boxes in order, as the tables were written above
+        for (int v = 0; v < kDepVariants; ++v)
+            for (int b = 0; b < nbox; ++b) c->dep_order[v].push_back(b);
+        if (deposit64_plan(c)) return bail(NTLP_ERR_CUDA);
+    }
     if (mixed) prepare_kernels_mixed(); else prepare_kernels64();
     if (c->blk_kb) prepare_interp_block();
     // the host vectors above are copied from: wait before they go out of scope
@@ -1168,7 +1199,7 @@ int droplets_upload(ntlp_ctx *c, int b, const ntlp_droplets *d) {
     h.n_uploaded = n;
     h.have_droplets = true;
     c->payload_valid = false;
-    return NTLP_OK;
+    return c->params.precision == NTLP_PREC_MIXED ? NTLP_OK : deposit64_plan(c);
 }
 
 int droplets_download(ntlp_ctx *c, int b, ntlp_droplets *d) {
@@ -1236,13 +1267,6 @@ int droplets_download(ntlp_ctx *c, int b, ntlp_droplets *d) {
     return NTLP_OK;
 }
 
-// kernels of one deposition: the tiles, plus the two cell-sum kernels when
-// a mixed box is dense
-int deposit_launches(const ntlp_ctx *c) {
-    if (c->params.precision != NTLP_PREC_MIXED) return 3;   // tiles, overflow, fold
-    return c->any_dense ? 5 : 3;   // tiles, overflow, fold (+ cell sums, dense nodes)
-}
-
 // whether the step interpolates over staged blocks
 bool staged_interp(const ntlp_ctx *c) {
     return c->blk_on && c->blk_kb > 0 && (!c->blk_auto || c->blk_pays);
@@ -1262,14 +1286,17 @@ int launch_deposit(ntlp_ctx *c) {
     cudaEvent_t e0 = phase_begin(c);
     const int v = c->dep_variant;
     c->overflow.begin();
-    if (c->params.precision == NTLP_PREC_MIXED)
+    if (c->params.precision == NTLP_PREC_MIXED) {
         launch_deposit_mixed(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
                              c->any_dense, c->overflow_list_d);
-    else
+        c->launches += c->any_dense ? 5 : 3;   // tiles, overflow, fold (+ cell sums, dense nodes)
+    } else {
+        const std::vector<TileRun> &runs = c->dep_runs[v];
         launch_deposit64(v, c->box_d, c->dep_tiles_d[v], c->n_dep_tiles[v], c->dp, c->stream, c->nbox,
-                         c->dep64_cap, c->overflow_list_d);
+                         runs.data(), (int)runs.size(), c->overflow_list_d);
+        c->launches += (int)runs.size() + 2;   // tiles, overflow, fold
+    }
     phase_end(c, PH_DEPOSIT, e0);
-    c->launches += deposit_launches(c);
     CK(cudaGetLastError());
     c->overflow.end();
     return NTLP_OK;
@@ -1836,7 +1863,8 @@ int ntlp_flux(ntlp_ctx *c, double *pflux, double *pmassflux, double *penegflux) 
 // instantiate it, unless the one held matches dt, nsteps and the variants
 static int build_graph(ntlp_ctx *c, double dt, int32_t it, int32_t nsteps) {
     if (c->gexec && c->g_dt == dt && c->g_nsteps == nsteps && c->g_dep == c->dep_variant &&
-        c->g_nt == c->nt_variant && c->g_blk == staged_interp(c) && c->g_kb == c->blk_kb)
+        c->g_nt == c->nt_variant && c->g_blk == staged_interp(c) && c->g_kb == c->blk_kb &&
+        c->g_runs == c->dep_runs[c->dep_variant])
         return NTLP_OK;
     if (c->gexec) {
         cudaGraphExecDestroy(c->gexec);
@@ -1871,6 +1899,7 @@ static int build_graph(ntlp_ctx *c, double dt, int32_t it, int32_t nsteps) {
     c->g_nt = c->nt_variant;
     c->g_blk = staged_interp(c);
     c->g_kb = c->blk_kb;
+    c->g_runs = c->dep_runs[c->dep_variant];
     return NTLP_OK;
 }
 
@@ -2127,7 +2156,7 @@ int ntlp_sub_immigrants(ntlp_ctx *c, const ntlp_droplets *d) {
     if (pull_boxes(c)) return NTLP_ERR_CUDA;     // also waits for the host copy of `total`
     h.n_uploaded = total;
     c->payload_valid = false;
-    return NTLP_OK;
+    return c->params.precision == NTLP_PREC_MIXED ? NTLP_OK : deposit64_plan(c);
 }
 
 int ntlp_sub_halo_get(ntlp_ctx *c, int32_t axis, double *out) {

@@ -467,7 +467,8 @@ __device__ __forceinline__ int tile_columns(const DevBox &B, int x0, int y0, int
 // latency of the merge: more warps help, fewer instructions do not.
 template <int TX, int TY, int TZ, int CAP>
 __global__ void __launch_bounds__(kDepositThreads, 3)
-k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams P, int *overflow_list) {
+k_deposit64(DevBox *boxes, const Tile *tiles, int first, int ntiles, const __grid_constant__ DevParams P,
+            int *overflow_list) {
     step_kernel_begin<false>();
     static_assert(TX * TY * TZ == kDepositThreads, "one thread per node of the tile");
     constexpr int COLS = (TX + 1) * (TY + 1), CSW = TZ + 2;
@@ -476,7 +477,7 @@ k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams 
     int *s_lid = (int *)(sm + V64_N * 8 * CAP);        // [CAP]
     int *s_t = s_lid + CAP;                            // [CAP]
     int *s_cs = s_t + CAP, *s_off = s_cs + COLS * CSW;
-    const Tile tl = tiles[blockIdx.x];
+    const Tile tl = tiles[blockIdx.x];   // of the run that starts at tile `first` of ntiles
     const DevBox &B = boxes[tl.box];
     const DevGrid &g = B.g;
     const int ntz = (g.nz2 + TZ - 1) / TZ, nty = (g.dny + TY - 1) / TY;
@@ -566,7 +567,7 @@ k_deposit64(DevBox *boxes, const Tile *tiles, const __grid_constant__ DevParams 
         // above the stage capacity: k_deposit64_overflow, which has the
         // registers of the global path
         if (threadIdx.x == 0)
-            overflow_put(overflow_list, gridDim.x, blockIdx.x, [](int *n) { return atomicAdd(n, 1); });
+            overflow_put(overflow_list, ntiles, first + blockIdx.x, [](int *n) { return atomicAdd(n, 1); });
         return;
     }
     if (!valid) return;

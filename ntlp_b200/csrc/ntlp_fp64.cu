@@ -450,11 +450,23 @@ void launch_payload64(DevBox *boxes, const Tile *tiles, int ntiles, const DevPar
 }
 
 template <int V, int C>
-static void dep64(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P, cudaStream_t st,
-                  int *overflow_list) {
+static void dep64_run(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P, cudaStream_t st,
+                      const TileRun &r, int *overflow_list) {
     constexpr int TX = kDepShape[V][0], TY = kDepShape[V][1], TZ = kDepShape[V][2], CAP = kDepCap64[C];
-    launch_step_kernel(k_deposit64<TX, TY, TZ, CAP>, ntiles, kDepositThreads,
-                       dep_smem_bytes(false, TX, TY, TZ) + CAP * kStage64, st, boxes, tiles, P, overflow_list);
+    launch_step_kernel(k_deposit64<TX, TY, TZ, CAP>, r.count, kDepositThreads,
+                       dep_smem_bytes(false, TX, TY, TZ) + CAP * kStage64, st, boxes, tiles + r.first, r.first,
+                       ntiles, P, overflow_list);
+}
+
+template <int V>
+static void dep64(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P, cudaStream_t st,
+                  const TileRun *runs, int nruns, int *overflow_list) {
+    constexpr int TX = kDepShape[V][0], TY = kDepShape[V][1], TZ = kDepShape[V][2];
+    for (int k = 0; k < nruns; ++k) {
+        const TileRun &r = runs[k];
+        (r.cap == 0 ? dep64_run<V, 0> : r.cap == 1 ? dep64_run<V, 1> : dep64_run<V, 2>)(boxes, tiles, ntiles, P, st,
+                                                                                      r, overflow_list);
+    }
     if (overflow_list)
         launch_step_kernel(k_deposit64_overflow<TX, TY, TZ>, ntiles < kOverflowBlocks ? ntiles : kOverflowBlocks,
                            kDepositThreads, 0, st, boxes, tiles, ntiles, P, overflow_list);
@@ -482,13 +494,11 @@ void prepare_kernels64() {
 }
 
 void launch_deposit64(int variant, DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P,
-                      cudaStream_t st, int nbox, int cap, int *overflow_list) {
+                      cudaStream_t st, int nbox, const TileRun *runs, int nruns, int *overflow_list) {
     if (ntiles <= 0) return;
     prepare_kernels64();
-    auto go = [&](auto dep) { dep(boxes, tiles, ntiles, P, st, overflow_list); };
-    if (variant == 1) go(cap == 0 ? dep64<1, 0> : cap == 1 ? dep64<1, 1> : dep64<1, 2>);
-    else if (variant == 2) go(cap == 0 ? dep64<2, 0> : cap == 1 ? dep64<2, 1> : dep64<2, 2>);
-    else go(cap == 0 ? dep64<0, 0> : cap == 1 ? dep64<0, 1> : dep64<0, 2>);
+    (variant == 1 ? dep64<1> : variant == 2 ? dep64<2> : dep64<0>)(boxes, tiles, ntiles, P, st, runs, nruns,
+                                                                  overflow_list);
     if (nbox > 0) launch_step_kernel(k_fold, dim3(kFoldBlocks, nbox, 6), 256, 0, st, boxes, overflow_list);
 }
 

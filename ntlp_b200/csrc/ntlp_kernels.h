@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "ntlp_dev.cuh"
+#include "ntlp_stage64.h"
 
 namespace ntlp {
 
@@ -79,19 +80,17 @@ void launch_update_rk3_64(int ilin, DevBox *boxes, const Tile *tiles, int ntiles
 void launch_payload64(DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P, double dt,
                       cudaStream_t st);
 // nbox: boxes whose periodic images are deposited as nodes, to be folded in (0:
-// none, the tiles on the periodic edges fold their own); cap: deposit64_cap;
-// overflow_list: as for the mixed deposition, or NULL (tiles above the
-// capacity then merge from global memory within the tiled kernel)
+// none, the tiles on the periodic edges fold their own); runs: the tiles by
+// their stage capacity, a launch each; overflow_list: as for the mixed
+// deposition, or NULL (tiles above the capacity then merge from global memory
+// within the tiled kernel)
 void launch_deposit64(int variant, DevBox *boxes, const Tile *tiles, int ntiles, const DevParams &P,
-                      cudaStream_t st, int nbox, int cap, int *overflow_list);
-// Droplets a tile stages (56 bytes each), by the density in droplets per cell:
-// a tile has about 500 cells, and one with more droplets merges from global
-// memory.  Three CTAs per SM up to 2 per cell, one CTA (but no global merge) up
-// to 7.  500,000 droplets at 1.8 per cell: 0.41 -> 0.18 ms, 1 M at 3.6 0.77 ->
-// 0.53, 700,000 at 6 0.59 -> 0.37.
-constexpr int kDepCap64[3] = {640, 1280, 3840};
-inline int deposit64_cap(double density) {
-    return density <= 1.05 || density > 7.0 ? 0 : (density <= 2.1 ? 1 : 2);
+                      cudaStream_t st, int nbox, const TileRun *runs, int nruns,
+                      int *overflow_list);
+// cells whose droplets a deposition tile stages
+inline int deposit_tile_cells(int variant) {
+    const int *t = kDepShape[variant];
+    return (t[0] + 1) * (t[1] + 1) * (t[2] + 1);
 }
 constexpr int kOverflowBlocks = 1184; // grid of the overflow tiles
 

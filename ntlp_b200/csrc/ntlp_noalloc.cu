@@ -240,7 +240,8 @@ extern "C" int ntlp_coupling_noalloc(const ntlp_grid *grid, const ntlp_params *p
     launch_sort(B_d, plan, st);
     launch_finish(B_d, 1, st);
     launch_payload64(B_d, drop_tiles, nd, dp, dt, st);
-    launch_deposit64(0, B_d, node_tiles, nn, dp, st, 0, deposit64_cap((double)n / (double)ncells), nullptr);
+    const TileRun all{0, nn, deposit64_cap(n, ncells, deposit_tile_cells(0))};
+    launch_deposit64(0, B_d, node_tiles, nn, dp, st, 0, &all, 1, nullptr);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         fprintf(stderr, "ntlp_coupling_noalloc: %s\n", cudaGetErrorString(e));
