@@ -240,7 +240,12 @@ extern "C" int ntlp_coupling_noalloc(const ntlp_grid *grid, const ntlp_params *p
     launch_sort(B_d, plan, st);
     launch_finish(B_d, 1, st);
     launch_payload64(B_d, drop_tiles, nd, dp, dt, st);
-    const TileRun all{0, nn, deposit64_cap(n, ncells, deposit_tile_cells(0))};
+    // The smallest stage at every density: half of the tiles of a box of this size
+    // lie on the periodic edges, and without image nodes they merge from global
+    // memory, through what L1 cache the stage leaves them.  The whole call with
+    // 640 / 1280 / 3840: 24^3 with 10,000 droplets 109 / 145 / 145 us, 20^3 with
+    // 30,000 246 / 316 / 315, with 60,000 403 / 558 / 519; 48^3 with 100,000 173 / 210 / 287.
+    const TileRun all{0, nn, 0};
     launch_deposit64(0, B_d, node_tiles, nn, dp, st, 0, &all, 1, nullptr);
     e = cudaGetLastError();
     if (e != cudaSuccess) {

@@ -40,14 +40,15 @@ def _bind(L):
     return f
 
 
-def test_noalloc_deposition_matches_ntlp_coupling():
+@pytest.mark.parametrize("n", [3000, 9000, 25000])     # 1.2, 3.7 and 10 droplets per cell
+def test_noalloc_deposition_matches_ntlp_coupling(n):
     import torch
     import ntlp_b200
 
     torch.cuda.set_device(0)
     params = gen.default_params(ilin=0)
-    case = small_case(params=params, n=3000, grid_n=(12, 10, 16))
-    s = ntlp_b200.DropletStep(case.grid, params, capacity=3000)
+    case = small_case(params=params, n=n, grid_n=(12, 10, 16))
+    s = ntlp_b200.DropletStep(case.grid, params, capacity=n)
     s.set_fields_ext(case.ext())
     s.set_droplets(case.droplets)
     s.particle_update_BE(case.dt, 1)
