@@ -41,8 +41,8 @@ UNITS = {
     "ntlp_checkpoint.cpp": [],
     "ntlp_subdomain.cu": [],
 }
-HEADERS = ["ntlp_math.h", "ntlp_hist.h", "ntlp_overflow.h", "ntlp_stage64.h", "ntlp_dev.cuh", "ntlp_kernels.h",
-           "ntlp_physics.cuh", "ntlp_deposit.cuh"]
+HEADERS = ["ntlp_math.h", "ntlp_hist.h", "ntlp_overflow.h", "ntlp_recip.h", "ntlp_stage64.h", "ntlp_dev.cuh",
+           "ntlp_kernels.h", "ntlp_physics.cuh", "ntlp_deposit.cuh"]
 
 
 def nvcc() -> str:

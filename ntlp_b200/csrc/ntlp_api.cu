@@ -36,6 +36,7 @@
 #include "ntlp_kernels.h"
 #include "ntlp_math.h"
 #include "ntlp_overflow.h"
+#include "ntlp_recip.h"
 #include "ntlp_stage64.h"
 
 using namespace ntlp;
@@ -708,28 +709,6 @@ void deposit_extents(DevGrid &g) {
     g.dny = g.sny + (g.periodic ? 2 : 0);
 }
 
-// The reciprocals of the FP64 deposition's denominators, dx, dy, dzu(k) and
-// dx dy dzu(k) as the device forms them: each correctly rounded.  False when
-// one of them has a significand of all ones or is outside 2^-100 .. 2^100,
-// where the division by reciprocal is not exact (div_by); the deposition
-// then divides.
-bool deposit_reciprocals(const DevGrid &g, const std::vector<double> &dzu, std::vector<double> &rec) {
-    auto ok = [](double d) {
-        const uint64_t m = ntlp_bits(d) & 0x000fffffffffffffULL;
-        return d > 0x1p-100 && d < 0x1p100 && m != 0x000fffffffffffffULL;
-    };
-    const size_t n = dzu.size();
-    rec.assign(2 * n, 1.0);
-    bool all = ok(g.dx) && ok(g.dy);
-    for (size_t k = 0; k < n; ++k) {
-        const double dV = g.dx * g.dy * dzu[k];
-        all = all && ok(dzu[k]) && ok(dV);
-        rec[k] = 1.0 / dzu[k];
-        rec[n + k] = 1.0 / dV;
-    }
-    return all;
-}
-
 // FP64 deposition: the runs of the tile tables by stage capacity, each box's
 // from the droplets it was given, not from its room for them (1 M droplets on
 // 128^3 with room for 6 M: 0.376 ms, as without; 0.959 by the room).  Where that
@@ -851,7 +830,8 @@ int create(int nbox, const ntlp_grid *grids, const ntlp_params *params, const in
         level_tables(h, grid->nnz, h.lut, B.g.lut_scale, h.rden);
         B.g.nlut = kLutPerLevel * nz2;
         double *rdep = (double *)B.g.rdzu;
-        if (!deposit_reciprocals(B.g, h.dzu, h.rdep)) B.g.rdzu = B.g.rdV = nullptr;
+        h.rdep.resize(2 * (size_t)nz3);
+        if (!deposit_reciprocals(g.dx, g.dy, h.dzu.data(), g.nnz, h.rdep.data())) B.g.rdzu = B.g.rdV = nullptr;
         if (mixed) {
             const size_t npad = (size_t)nz2 * B.g.ny5 * B.g.nx5 + 2 * kF32Guard;
             if (cudaMemsetAsync((void *)(B.f4 - kF32Guard), 0, npad * sizeof(float4), c->stream) ||
