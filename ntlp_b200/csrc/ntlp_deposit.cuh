@@ -457,14 +457,16 @@ __device__ __forceinline__ int tile_columns(const DevBox &B, int x0, int y0, int
 // FP64 tiles (z fastest); tile shapes 2x4x32, 4x4x16 and 2x2x64 nodes are
 // instantiated (autotuned).
 //
-// Bound by the FP64 pipe and the shared-memory pipe together: a node merges
-// about 8 droplets at one per cell, each of them 10 terms of a multiply, a
-// division, a multiply and a subtraction.  The trilinear weights (6 a droplet)
-// are formed while staging, not 3 per node, the divisions by the cell volume
-// take div_by, and the merge keeps its 8 list heads in registers.
-// 16.8 M droplets on 256^3: 8.00 -> 4.15 ms; 1 M on 128^3: 0.71 -> 0.39 ms, where
-// the edge tiles' merges from global memory counted most.  The rest is the
-// latency of the merge: more warps help, fewer instructions do not.
+// Bound by the latency of the merge: a node merges about 8 droplets at one per
+// cell, each of them 10 terms of a multiply, a division, a multiply and a
+// subtraction, and half of a warp's lanes wait for the longest list.  Issue is at
+// 52%, the L1 data pipe at 58%, the FP64 pipe at 29% with 21 warps on an SM
+// (profiles/k_deposit64_2M_droplets_128cube.md); more warps help, fewer
+// instructions do not.  The trilinear weights (6 a droplet) are formed while
+// staging, not 3 per node, the divisions by the cell volume take div_by, and the
+// merge keeps its 8 list heads in registers.  16.8 M droplets on 256^3: 7.90 ->
+// 4.04 ms; 1 M on 128^3: 0.71 -> 0.375 ms, where the edge tiles' merges from global
+// memory counted most.
 template <int TX, int TY, int TZ, int CAP>
 __global__ void __launch_bounds__(kDepositThreads, 3)
 k_deposit64(DevBox *boxes, const Tile *tiles, int first, int ntiles, const __grid_constant__ DevParams P,

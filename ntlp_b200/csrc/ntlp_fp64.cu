@@ -99,15 +99,16 @@ __device__ __forceinline__ void lagrange6(double x, const double xn[6], int firs
 
 // uf_interp, particles.f90:554-765.
 //
-// Bound by instruction issue and the FP64 pipe: 216 points of 3 multiplies and
-// an add for each of 5 fields, 4320 operations that the order of the reference
-// does not let share anything.  What is left to save is around them: a point
+// Bound by the latency of its loads and of dependent FP64 instructions, with two
+// pipes half busy: 216 points of 3 multiplies and an add for each of 5 fields,
+// 4320 operations that the order of the reference does not let share anything.  What is left to save is around them: a point
 // is one 32-byte load and one of w, at 32-bit offsets, and the j and i loops
 // are unrolled so that no weight moves between registers (k stays rolled):
 // 12298 -> 9218 instructions a warp, 11.9 -> 10.1 ms for 16.8 M droplets at 16
-// warps per SM (12 and 20 are slower).  The FP64 pipe is then at 49% and the
-// L1 data pipe at 59%.  Mapping CTAs to blocks of cells raises the L1 hits from
-// 23% to 93% and is no faster: the L2 latency is hidden.
+// warps per SM (12 and 20 are slower).  The FP64 pipe is then at 49%, the L1
+// data pipe at 66% and issue at 41%
+// (profiles/k_interp64_2M_droplets_128cube.md).  Mapping CTAs to blocks of cells
+// raises the L1 hits from 24% to 93% and is no faster: the L2 latency is hidden.
 __device__ void interp6_64(const DevBox &B, double x1, double x2, double x3, Interp &o, int &bad) {
     const DevGrid &g = B.g;
     const int nnz = g.nnz;

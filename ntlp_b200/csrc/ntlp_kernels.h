@@ -36,7 +36,7 @@ constexpr int kNtValues[kNtVariants] = {128, 256};
 // completed and its writes are visible.  Nothing runs earlier than before
 // but the placement.
 // A kernel that fills the SMs' shared memory (EARLY false: the staged
-// interpolation, the mixed deposition) lets nothing in before it has
+// interpolation, the tiled depositions) lets nothing in before it has
 // completed: its successor would run on with the L1 cache that those CTAs left
 // it (16.8 M droplets, update: 5.76 ms without, 5.98 with; overflow tiles of the
 // spray case: 6.8 and 15 ms).  10,000 droplets on 32^3: update 47 -> 43, sort 29 ->
@@ -112,13 +112,14 @@ void prepare_interp_block();         // kernel attributes, once per device
 // 3.6 with 4 / 8 / 16: 0.331 / 0.326 / 0.341 ms, 2 M at 29 0.624 / 0.649 / 0.786 ms.
 inline int interp_block_kb(double density) { return density < 3.0 ? 16 : (density < 6.0 ? 8 : 4); }
 // Whether the staged blocks beat the per-droplet kernel (the same bits): a block
-// stages 3.2 KB of fields per cell column and 16 levels whether it holds
+// of 16 levels stages 2.4 KB of fields per cell column whether it holds
 // droplets or not, and its CTAs take turns of latency that a small box cannot
 // overlap.  Update phase, per droplet against staged: 0.063 against 0.143 ms (10,000
 // droplets, 0.005 per cell), 0.275 against 0.341 (500,000, 0.23), 3.27 against
 // 3.53 (8 M, 0.47), 0.121 against 0.126 (250,000, 0.91), 0.190 against 0.188 (500,000,
 // 1.8); 0.737 against 0.732 (2 M, 0.93), 5.83 against 5.61 (16.7 M, 0.98), 1.28 against
 // 1.18 (4 M, 1.9), 0.637 against 0.624 (2 M, 29); 0.660 against 0.686 (2 M, 56).
+// Both rules go by the context's room for droplets; all were measured full.
 inline bool interp_staged_pays(double density, double droplets) {
     return density >= 0.75 && density < 40.0 && droplets >= 1e6;
 }

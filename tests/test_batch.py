@@ -174,7 +174,7 @@ def test_autotune_changes_no_result(precision):
 
 @pytest.mark.parametrize("precision", [abi.NTLP_PREC_FP64, abi.NTLP_PREC_MIXED])
 def test_dense_box_in_a_batch(precision):
-    # a box of ~100 droplets per cell (large-cell ranking; mixed: per-cell
+    # a box of ~100 droplets per cell (long rank loops; mixed: per-cell
     # sums) beside sparse boxes: every box equals itself alone, eager and graph
     import ntlp_b200
     params = gen.default_params(ilin=0, precision=precision)

@@ -85,8 +85,8 @@ def test_be_fp64_bitexact(ilin, icase):
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_dense_cells(precision):
-    # ~100 droplets per cell: cells above the insertion-sort size are put in
-    # lid order by ranking, and every tile overflows the deposition stage
+    # ~100 droplets per cell: each counts the smaller lids of many others, and
+    # every tile overflows the deposition stage
     params = gen.default_params(ilin=0)
     case = small_case(params=params, n=20000, grid_n=(4, 4, 6))
     p = dict(params, precision=abi.NTLP_PREC_MIXED if precision == "mixed" else abi.NTLP_PREC_FP64)

@@ -1,6 +1,6 @@
-"""Mixed deposition tiles above their stage's capacity (768 droplets): taken in
-slabs of levels, or a level from global memory, against the per-cell sums that
-boxes of large capacity use.  The sources are the same bits."""
+"""Mixed deposition tiles above their stage's capacity (768 droplets), which the
+overflow kernel merges from global memory, against the per-cell sums that boxes of
+large capacity use.  The sources are the same bits."""
 import numpy as np
 import pytest
 
@@ -11,14 +11,14 @@ from ntlp_b200 import generator as gen
 
 
 @pytest.mark.parametrize("grid_n,n", [
-    ((9, 9, 70), 30_000),     # slabs of many levels, ragged tiles in every direction
-    ((5, 3, 40), 9_000),      # about 9 a cell
-    ((4, 5, 33), 14_000),     # slabs of a level or two
-    ((2, 2, 3), 2_500),       # one level's cells exceed the stage
+    ((9, 9, 70), 30_000),     # 4.2 a cell: ragged tiles in every direction, above the stage and below
+    ((5, 3, 40), 9_000),      # 9 a cell
+    ((4, 5, 33), 14_000),     # 14 a cell
+    ((2, 2, 3), 2_500),       # 69 a cell, the smallest grid
 ])
 @pytest.mark.gpu
 @pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")
-def test_slabs_match_cell_sums(grid_n, n):
+def test_overflow_tiles_match_cell_sums(grid_n, n):
     import ntlp_b200
     params = dict(gen.default_params(icase=0), precision=abi.NTLP_PREC_MIXED)
     case = small_case(params=params, n=n, grid_n=grid_n)
@@ -42,4 +42,4 @@ def test_fold_of_thin_boxes(grid_n):
     """Boxes whose border nodes are all or most of them, and more than one round of
     the fold's blocks: the images folded by a kernel of its own against the folded
     cell sums.  The sources are the same bits."""
-    test_slabs_match_cell_sums(grid_n, 3_000)
+    test_overflow_tiles_match_cell_sums(grid_n, 3_000)
